@@ -118,3 +118,17 @@ def test_sums_of_many_columns(lib, rows, cols, offset):
     expected = base.copy()
     expected[offset:] += x.sum(axis=0)
     close(host(tout), expected, 1e-5)
+
+
+def test_gelu_slope_of_large_values(lib):
+    """The slope in the product's epilogue far out: one to the right, zero to the
+    left, for every value whose square is finite (the TF32 product's bound)."""
+    m, k, n = 256, 128, 64
+    rng = np.random.RandomState(3)
+    w, dy = rng.randn(k, n) / np.sqrt(n), rng.randn(m, n)
+    hidden = np.exp(rng.uniform(np.log(5.0), np.log(1.8e19), (m, k)))
+    hidden *= rng.choice([-1.0, 1.0], (m, k))
+    tw, tdy, th, tdh = map(dev, (w, dy, hidden, np.zeros((m, k))))
+    assert lib.vitb200_k_gemm_backward_gelu(ptr(tw), ptr(tdy), ptr(th), ptr(tdh), None,
+                                            size(m), size(k), size(n), TF32, None) == 0
+    close(host(tdh), np.where(hidden > 0, dy @ w.T, 0.0), 2e-3)

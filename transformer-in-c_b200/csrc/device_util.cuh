@@ -168,8 +168,8 @@ __device__ __forceinline__ float gelu_complement(float x, float x2) {
     return __fdividef(1.0f, 1.0f + e);
 }
 
-// The same function as x (1 - r): absolute error about 2e-7, a fifth of the
-// instructions.  Used where the GELU shares a kernel with a matrix product and
+// The same function as x (1 - r): absolute error 3.9e-7 at most (5e-8 rms over
+// normally distributed values), a fifth of the instructions.  Used where the GELU shares a kernel with a matrix product and
 // instruction issue, not memory, is the limit.
 __device__ __forceinline__ float gelu_value_fast(float x) {
     return x * (1.0f - gelu_complement(x, x * x));
@@ -184,14 +184,18 @@ __device__ __forceinline__ float gelu_slope(float x) {
 }
 
 
-// gelu_slope with the same r (absolute error about 3e-7), for the epilogue of the
-// product that feeds a GELU's backward pass:
+// gelu_slope with the same r, for the epilogue of the product that feeds a GELU's
+// backward pass (absolute error 2.0e-6 at most, near x = -5; 5e-8 rms over normally
+// distributed values):
 //   0.5 (1 + t) + 0.5 x (1 - t^2) u' = h + 2 r h x u',  h = 1 - r
+// From |x| = 16 on r h is zero and x^2 stays at 256, so that the factor beside it
+// is finite for every x whose square is (x u' alone overflows from 1.2e13 on).
 __device__ __forceinline__ float gelu_slope_fast(float x) {
     const float x2 = x * x;
     const float r = gelu_complement(x, x2);
     const float h = 1.0f - r;
-    const float slope = x * fmaf(6.0f * kGeluScale * kGeluCubic, x2, 2.0f * kGeluScale);
+    const float slope = x * fmaf(6.0f * kGeluScale * kGeluCubic, fminf(x2, 256.0f),
+                                 2.0f * kGeluScale);
     return fmaf(h * r, slope, h);
 }
 
