@@ -132,3 +132,24 @@ def test_gelu_slope_of_large_values(lib):
     assert lib.vitb200_k_gemm_backward_gelu(ptr(tw), ptr(tdy), ptr(th), ptr(tdh), None,
                                             size(m), size(k), size(n), TF32, None) == 0
     close(host(tdh), np.where(hidden > 0, dy @ w.T, 0.0), 2e-3)
+
+
+@pytest.mark.parametrize("rows,cols", [(64, 24600), (128, 50432), (700, 16384),
+                                       (2049, 4096), (2048, 6400), (10000, 4096)])
+def test_error_of_sums_of_many_columns(lib, rows, cols):
+    """No larger than what the narrow sums' kernel leaves: lanes of a 32nd of a slice's
+    rows, a tree of five levels, an addition per slice.  Along a row of L additions
+    the running sum's square is half the result's on average, in a tree every level's
+    is the result's.  Rounding a value of significand s leaves 2^-24 / (sqrt(3) s) of
+    it, over the significands of normal sums 0.44 x 2^-24; the bound takes 0.475."""
+    rng = np.random.RandomState(rows)
+    x = rng.randn(rows, cols).astype(np.float32)
+    tx, tout = dev(x), torch.zeros(cols, device="cuda")
+    lib.vitb200_k_column_sums(ptr(tx), ptr(tout), size(rows), size(cols), None)
+    exact = x.astype(np.float64).sum(axis=0)
+    error = np.linalg.norm(host(tout) - exact) / np.linalg.norm(exact)
+    strips = (cols + 127) // 128
+    slices = max(1, min((296 + strips - 1) // strips, (rows + 127) // 128))
+    row = np.ceil(rows / slices / 32)
+    bound = 2.0 ** -24 * 0.475 * np.sqrt(row / 2 + 5 + slices / 2)
+    assert error <= bound, (error, bound)

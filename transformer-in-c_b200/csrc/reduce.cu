@@ -73,43 +73,92 @@ column_sums_kernel(const float *__restrict__ in, float *__restrict__ out,
 }
 
 // Many columns, few rows (the positional gradients: a row per image, a column per
-// token and feature): a thread owns four columns and walks its slice of the rows
-// with eight loads in flight, with nothing to fold.  Bound by memory; the kernel
-// above spends its time there on 32 row lanes that find two rows each, and on
-// their fold: 64 rows of 393600 columns (101 MB, 15 us at the copy rate) took it
-// 67 us, this one 17 (512 rows of 50432 columns 24.5 and 18.7, 128 rows 19.8 and 8.7).
-constexpr int kStripThreads = 128;
-// 2048 rows of 6400 columns 14.4 us there and 9.8 here; the bias gradients, with at
-// most a few thousand columns and many more rows, stay there.
+// token and feature): eight row lanes with eight loads in flight each, where the
+// kernel above has 32 lanes that find two rows each and a fold in five steps.
+// Bound by memory: 64 rows of 393600 columns (101 MB, 15 us at the copy rate) take the
+// kernel above 72 us, this one 25; 2048 rows of 50432 columns 80 and 72, of 6400
+// columns 25 and 18.
+//
+// The rows are added up as trees (eight loads, then eight lanes), so that a sum's
+// error is no larger than there (2-norm against 64 bits, normal values: 0.7e-7 and
+// 0.7e-7, 1.6e-7 and 1.0e-7, 1.0e-7 and 1.0e-7 for the three; one row after the other
+// gave 1.1e-7, 2.5e-7 and 2.0e-7 in the same time).  The bound on the registers keeps
+// the eight loads together: without it 25600 x 4096 takes 96 us instead of 74.
+constexpr int kStripLanes = 8;
+// From this many columns on, bias gradients as wide as that among them.  At 4096 it
+// takes 14 us for 2049 rows (there 20) and 74 for 25600 (91); narrower sums have many
+// more rows than columns and stay above.
 constexpr size_t kStripColumns = 4096;
 
-__global__ void __launch_bounds__(kStripThreads)
+// Slices of the rows: what fills two blocks per SM, in whole rounds of them.  (Four
+// are resident, but every slice is one more addition in a row for each sum: at four
+// 2049 x 4096 had 1.07 of the error above, and is no faster.)
+size_t strip_slices(size_t rows, size_t strips) {
+    const size_t round = size_t(device_sm_count()) * 2;
+    const size_t loads = 8 * kStripLanes;   // rows of a block's round of loads
+    const size_t most = std::min<size_t>(
+        std::min<size_t>((rows + loads - 1) / loads, 65535),
+        std::max<size_t>(4, (round + strips - 1) / strips));
+    size_t best = 1;
+    double least = 0.0;
+    for (size_t slices = 1; slices <= most; ++slices) {
+        const double turns = double((strips * slices + round - 1) / round);
+        const size_t rows_each = (rows + slices - 1) / slices;
+        const double time =
+            turns * double((rows_each + loads - 1) / loads) + 0.02 * double(slices);
+        if (slices == 1 || time < least) {
+            best = slices;
+            least = time;
+        }
+    }
+    return best;
+}
+
+__device__ __forceinline__ float4 add4(const float4 &a, const float4 &b) {
+    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+
+__device__ __forceinline__ float4 tree8(const float4 (&v)[8]) {
+    return add4(add4(add4(v[0], v[1]), add4(v[2], v[3])),
+                add4(add4(v[4], v[5]), add4(v[6], v[7])));
+}
+
+__global__ void __launch_bounds__(kLanesX *kStripLanes, 4)
 column_strips_kernel(const float *__restrict__ in, float *__restrict__ out,
                      size_t rows, size_t cols, size_t ld, size_t rows_per_block) {
     grid_dependency_wait();
     grid_dependency_release();
-    constexpr int R = 8;
-    const size_t col = (size_t(blockIdx.x) * kStripThreads + threadIdx.x) * 4;
+    __shared__ float4 partial[kStripLanes][kLanesX];
+    const size_t col = (size_t(blockIdx.x) * kLanesX + threadIdx.x) * 4;
     const size_t row_begin = size_t(blockIdx.y) * rows_per_block;
     const size_t row_end = min(rows, row_begin + rows_per_block);
-    if (col >= cols || row_begin >= row_end) {
-        return;
-    }
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 sum = zero;
-    for (size_t row = row_begin; row < row_end; row += R) {
-        float4 v[R];
+    if (col < cols) {
+        for (size_t row = row_begin + threadIdx.y; row < row_end;
+             row += 8 * kStripLanes) {
+            float4 v[8];
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            v[r] = row + r < row_end
-                ? __ldcs(reinterpret_cast<const float4 *>(in + (row + r) * ld + col))
-                : zero;
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            sum.x += v[r].x; sum.y += v[r].y; sum.z += v[r].z; sum.w += v[r].w;
+            for (int r = 0; r < 8; ++r) {
+                const size_t mine = row + r * kStripLanes;
+                v[r] = mine < row_end
+                    ? __ldcs(reinterpret_cast<const float4 *>(in + mine * ld + col))
+                    : zero;
+            }
+            sum = add4(sum, tree8(v));
         }
     }
+    partial[threadIdx.y][threadIdx.x] = sum;
+    __syncthreads();
+    if (threadIdx.y != 0 || col >= cols || row_begin >= row_end) {
+        return;
+    }
+    float4 lanes[kStripLanes];
+#pragma unroll
+    for (int y = 0; y < kStripLanes; ++y) {
+        lanes[y] = partial[y][threadIdx.x];
+    }
+    sum = tree8(lanes);
     float *target = out + col;
     if ((reinterpret_cast<size_t>(target) & 15) == 0) {
         asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::
@@ -198,15 +247,11 @@ void launch_column_sums(const float *in, float *out, size_t rows, size_t cols,
     }
     const bool vec = cols % 4 == 0 && ld % 4 == 0;
     if (vec && cols >= kStripColumns) {
-        const size_t strips = (cols / 4 + kStripThreads - 1) / kStripThreads;
-        // Eight rows at least in a slice, about a thousand threads per SM in all.
-        const size_t wanted =
-            (size_t(device_sm_count()) * 1024 / kStripThreads + strips - 1) / strips;
-        const size_t slices = std::min<size_t>(std::min<size_t>(wanted, (rows + 7) / 8), 65535);
-        launch_streamed(column_strips_kernel,
-                        dim3(unsigned(strips), unsigned(slices)), kStripThreads, stream,
-                        4 * rows * cols, in, out, rows, cols, ld,
-                        (rows + slices - 1) / slices);
+        const size_t strips = (cols / 4 + kLanesX - 1) / kLanesX;
+        const size_t slices = strip_slices(rows, strips);
+        launch_streamed(column_strips_kernel, dim3(unsigned(strips), unsigned(slices)),
+                        dim3(kLanesX, kStripLanes), stream, 4 * rows * cols, in, out,
+                        rows, cols, ld, (rows + slices - 1) / slices);
         ++g_kernel_launches;
         return;
     }
