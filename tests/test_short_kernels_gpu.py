@@ -153,3 +153,29 @@ def test_error_of_sums_of_many_columns(lib, rows, cols):
     row = np.ceil(rows / slices / 32)
     bound = 2.0 ** -24 * 0.475 * np.sqrt(row / 2 + 5 + slices / 2)
     assert error <= bound, (error, bound)
+
+
+def split_row_bound(m, n, k):
+    """2-norm error of a weight gradient [m, n] over k rows, as sums of at least 128
+    rows in slices of the reduction, two tiles of 64 x 64 per SM; per addition as in
+    test_error_of_sums_of_many_columns."""
+    tiles = -(-m // 64) * -(-n // 64)
+    slices = max(1, min(-(-296 // tiles), -(-k // 128)))
+    rows = -(-(-(-k // slices)) // 16) * 16
+    return 2.0 ** -24 * 0.475 * np.sqrt((min(rows, k) + slices) / 2)
+
+
+@pytest.mark.parametrize("m,k,n", [
+    (8200, 9, 128), (8625, 1, 256), (10007, 16, 128), (20000, 4, 256), (12000, 12, 1024),
+    (9000, 4, 4),
+])
+def test_error_of_thin_weight_gradients(lib, m, k, n):
+    rng = np.random.RandomState(m + n)
+    x, dy = (rng.randn(m, c).astype(np.float32) for c in (k, n))
+    tx, tdy, tw = dev(x), dev(dy), dev(rng.randn(k, n))
+    tdx, tdw = torch.zeros(m, k, device="cuda"), torch.zeros(k, n, device="cuda")
+    assert lib.vitb200_k_gemm_backward(ptr(tx), ptr(tw), ptr(tdy), ptr(tdx), ptr(tdw),
+                                       size(m), size(k), size(n), FP32, None) == 0
+    exact = x.astype(np.float64).T @ dy.astype(np.float64)
+    error = np.linalg.norm(host(tdw) - exact) / np.linalg.norm(exact)
+    assert error <= split_row_bound(k, n, m), (error, split_row_bound(k, n, m))

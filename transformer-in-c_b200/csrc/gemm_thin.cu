@@ -16,7 +16,7 @@
 //
 // Measured against the tiled FMA kernel, 4 features: [100352,4]x[4,256] forward
 // 67 -> 18.7 us (104 MB: 16 at the copy rate), input gradient 61 -> 22.8, weight
-// gradient 76 -> 26.3; [65536,4]x[4,384] 67 -> 18.3, 59 -> 24.7, 79 -> 30.9.
+// gradient 76 -> 21.9; [65536,4]x[4,384] 67 -> 18.3, 59 -> 24.7, 79 -> 20.9.
 #include "device_util.cuh"
 #include "gemm.h"
 #include "kernels.h"
@@ -29,6 +29,13 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kMaxGroups = kThreads;       // float4 column groups of the wide extent
+// The weight gradient's blocks, one per SM: every block is one more addition in a row
+// for each of its sums.  With up to 444 blocks of 256 threads [10007,16]^T [10007,128]
+// had an error of 3.2e-7 (2-norm against 64 bits; 2.7e-7 on the tiles the kernel stands
+// in for), this way 2.3e-7, and [65536,4]^T [65536,384] 4.0e-7 (6.7e-7), now 2.7e-7.
+// The 128 registers leave room for no more threads, so that one block fills the SM and
+// no second, half-empty turn of blocks follows: 17.3 -> 13.3 us and 30.3 -> 20.9.
+constexpr int kWeightThreads = 512;
 // Below this many rows the tiles of the general kernel are as fast.
 constexpr int kMinimumRows = 8192;
 
@@ -37,6 +44,10 @@ __device__ __forceinline__ void fma4(float4 &sum, float x, const float4 &w) {
     sum.y = fmaf(x, w.y, sum.y);
     sum.z = fmaf(x, w.z, sum.z);
     sum.w = fmaf(x, w.w, sum.w);
+}
+
+__device__ __forceinline__ void add(float4 &sum, const float4 &v) {
+    sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
 }
 
 // The first k of KM values; zeros beyond.
@@ -184,15 +195,15 @@ thin_input_gradient_kernel(const float *__restrict__ a, const float *__restrict_
 }
 
 template <int MM>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kWeightThreads, 1)
 thin_weight_gradient_kernel(const float *__restrict__ a, const float *__restrict__ b,
                             float *c, int m, unsigned k, unsigned groups, size_t lda,
                             size_t ldb, size_t ldc, bool vector) {
     grid_dependency_wait();
     grid_dependency_release();
     constexpr int R = MM <= 4 ? 8 : (MM <= 8 ? 4 : 2);
-    __shared__ float4 fold[kThreads];
-    const unsigned slices = kThreads / groups;
+    __shared__ float4 fold[kWeightThreads], folded[kWeightThreads];
+    const unsigned slices = kWeightThreads / groups;
     const unsigned slice = threadIdx.x / groups, group = threadIdx.x % groups;
     const bool live = slice < slices;
     float4 sums[MM];
@@ -220,21 +231,29 @@ thin_weight_gradient_kernel(const float *__restrict__ a, const float *__restrict
             }
         }
     }
-    // The block's slices together, then one reduction into C per column group.
+    // The block's slices together, a square root of them at a time, then one
+    // reduction into C per column group.
+    unsigned lanes = 1;
+    while (lanes * lanes < slices) {
+        ++lanes;
+    }
 #pragma unroll
     for (int i = 0; i < MM; ++i) {
         if (i < m) {
-            if (i > 0) {
-                __syncthreads();
-            }
             fold[threadIdx.x] = sums[i];
             __syncthreads();
+            if (slice < lanes) {
+                float4 total = fold[threadIdx.x];
+                for (unsigned s = slice + lanes; s < slices; s += lanes) {
+                    add(total, fold[s * groups + group]);
+                }
+                folded[threadIdx.x] = total;
+            }
+            __syncthreads();
             if (slice == 0) {
-                float4 total = fold[group];
-                for (unsigned s = 1; s < slices; ++s) {
-                    const float4 other = fold[s * groups + group];
-                    total.x += other.x; total.y += other.y;
-                    total.z += other.z; total.w += other.w;
+                float4 total = folded[group];
+                for (unsigned s = 1; s < lanes; ++s) {
+                    add(total, folded[s * groups + group]);
                 }
                 asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::
                                  "l"(c + i * ldc + 4 * group),
@@ -331,9 +350,9 @@ bool launch_gemm_thin(const FmaGemm &g, cudaStream_t stream) {
         }
         const bool vector = g.m % 4 == 0 && fits(lda) && aligned(g.a);
         const size_t bytes = 4 * size_t(g.k) * (g.n + g.m);
-        const unsigned grid = row_blocks(g.k, 4 * (kThreads / groups), 3);
+        const unsigned grid = row_blocks(g.k, 4 * (kWeightThreads / groups), 1);
         auto launch = [&](auto kernel) {
-            status = launch_streamed(kernel, grid, kThreads, stream, bytes, g.a, g.b,
+            status = launch_streamed(kernel, grid, kWeightThreads, stream, bytes, g.a, g.b,
                                      g.c, g.m, unsigned(g.k), groups, lda, ldb, ldc,
                                      vector);
         };
