@@ -156,8 +156,8 @@ def test_error_of_sums_of_many_columns(lib, rows, cols):
 
 
 def split_row_bound(m, n, k):
-    """2-norm error of a weight gradient [m, n] over k rows, as sums of at least 128
-    rows in slices of the reduction, two tiles of 64 x 64 per SM; per addition as in
+    """2-norm error of a gradient [m, n], sums of k terms, in slices of at least 128
+    of them, as many as make two tiles of 64 x 64 per SM; per addition as in
     test_error_of_sums_of_many_columns."""
     tiles = -(-m // 64) * -(-n // 64)
     slices = max(1, min(-(-296 // tiles), -(-k // 128)))
@@ -179,3 +179,22 @@ def test_error_of_thin_weight_gradients(lib, m, k, n):
     exact = x.astype(np.float64).T @ dy.astype(np.float64)
     error = np.linalg.norm(host(tdw) - exact) / np.linalg.norm(exact)
     assert error <= split_row_bound(k, n, m), (error, split_row_bound(k, n, m))
+
+
+@pytest.mark.parametrize("m,k,n", [
+    (4329, 96, 288), (1972, 128, 1024), (18321, 32, 256), (2905, 32, 1536),
+    (4423, 64, 1024), (700, 1000, 300), (65, 33, 4000),
+])
+def test_error_of_accumulated_gradients(lib, m, k, n):
+    """Both gradients of an FP32 product where its slices decide the error."""
+    rng = np.random.RandomState(m + n)
+    x, w, dy = (rng.randn(*s).astype(np.float32) for s in ((m, k), (k, n), (m, n)))
+    tx, tw, tdy = map(dev, (x, w, dy))
+    tdx, tdw = torch.zeros(m, k, device="cuda"), torch.zeros(k, n, device="cuda")
+    assert lib.vitb200_k_gemm_backward(ptr(tx), ptr(tw), ptr(tdy), ptr(tdx), ptr(tdw),
+                                       size(m), size(k), size(n), FP32, None) == 0
+    x, w, dy = (a.astype(np.float64) for a in (x, w, dy))
+    for found, exact, bound in ((tdx, dy @ w.T, split_row_bound(m, k, n)),
+                                (tdw, x.T @ dy, split_row_bound(k, n, m))):
+        error = np.linalg.norm(host(found) - exact) / np.linalg.norm(exact)
+        assert error <= bound, (error, bound)

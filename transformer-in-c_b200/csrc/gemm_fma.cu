@@ -34,6 +34,7 @@
 #include "device_util.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <cstdint>
 
 namespace vitb200 {
@@ -520,28 +521,55 @@ constexpr int kSmallestTile = kTileCount - 1;
 struct FmaPlan {
     int tile = 0;
     int slices = 1;
+    bool cluster = false;   // the slices of a tile meet in a cluster, else in C
     double clocks = 0.0;
 };
 
+int slice_length(int k, int slices) {
+    return ((k + slices - 1) / slices + 15) / 16 * 16;
+}
+
+// Slices that 64 x 64 tiles take to make up two CTAs per SM, of 128 terms at least.
+int reference_slices(int m, int n, int k) {
+    const long long tiles = ((m + 63LL) / 64) * ((n + 63LL) / 64);
+    const long long two = 2LL * device_sm_count();
+    const int wanted = int(std::min((two + tiles - 1) / tiles, (k + 127LL) / 128));
+    const int each = slice_length(k, std::max(1, wanted));
+    return each ? (k + each - 1) / each : 1;
+}
+
+// Additions that follow one another in a sum: a slice's terms, then the slices.
+long long additions(int k, int slices) {
+    return std::min(k, slice_length(k, slices)) + (long long)slices;
+}
+
 // Picks the plan with the smallest estimate: the longer of what one CTA takes
 // by itself and what an SM takes for all the CTAs it gets, plus the fixed part
-// and what combining slices costs.
-FmaPlan plan_product(int m, int n, int k, bool split) {
+// and what combining slices costs.  reduce: C is added to, so that slices may
+// meet there (weight gradients); cluster: the smallest tile's slices meet in a
+// cluster (forward products and input gradients).  Plans whose sums take more
+// than `longest` additions in a row are left out.
+FmaPlan plan_product(int m, int n, int k, bool reduce, bool cluster, long long longest) {
     const double sms = double(device_sm_count());
+    const int reference = reference_slices(m, n, k);
     FmaPlan best;
     for (int t = 0; t < kTileCount; ++t) {
         const Tile &tile = kTiles[t];
         const double count = double((m + tile.rows - 1) / tile.rows) *
                              double((n + tile.cols - 1) / tile.cols);
-        // Slices: for weight gradients powers of two and as many as give every
-        // SM one to eight CTAs, added up by reductions in L2; otherwise a
-        // cluster of 2, 4 or 8 for the smallest tile.
-        const int choices = split ? 16 : (t == kSmallestTile ? 4 : 1);
+        // Slices that meet in C: powers of two, as many as give every SM one to
+        // eight CTAs, and the reference; in a cluster 2, 4 or 8.
+        const bool in_cluster = cluster && t == kSmallestTile;
+        const int choices = in_cluster ? 4 : (reduce ? 17 : 1);
         for (int choice = 0; choice < choices; ++choice) {
             const int slices = choice < 8 ? 1 << choice
-                : std::max(1, int((choice - 7) * sms / count));
-            const int per_slice = ((k + slices - 1) / slices + 15) / 16 * 16;
-            if (slices > 1 && per_slice < (split ? 32 : 16)) {
+                : (choice == 16 ? reference
+                                : std::max(1, int((choice - 7) * sms / count)));
+            const int per_slice = slice_length(k, slices);
+            if (slices > 1 && per_slice < (in_cluster ? 16 : 32)) {
+                continue;
+            }
+            if (additions(k, slices) > longest) {
                 continue;
             }
             const double work = double(tile.rows) * tile.cols * per_slice;
@@ -549,16 +577,31 @@ FmaPlan plan_product(int m, int n, int k, bool split) {
             double clocks = std::max(work / tile.alone, per_sm * work / tile.full) +
                             tile.fixed;
             if (slices > 1) {
-                clocks += split ? double(m) * n * slices / 1500.0 : 2200.0;
+                clocks += in_cluster ? 2200.0 : double(m) * n * slices / 1500.0;
             }
             if (best.clocks == 0.0 || clocks < best.clocks) {
                 best.tile = t;
                 best.slices = slices;
+                best.cluster = in_cluster;
                 best.clocks = clocks;
             }
         }
     }
     return best;
+}
+
+// The plan of a product that adds to C.  Its slices bound the rounding error, which
+// grows with the square root of the additions in a row: no more of them than the
+// reference takes.  (In one chain of 288 the input gradient [4329,288] x [288,96] had an
+// error of 3.0e-7, in slices of 96 1.8e-7.)  An input gradient is cut that way only
+// where its ordinary plan is longer.
+FmaPlan plan_addition(int m, int n, int k, bool input_gradient) {
+    const long long longest = additions(k, reference_slices(m, n, k));
+    FmaPlan plan = plan_product(m, n, k, !input_gradient, input_gradient, LLONG_MAX);
+    if (additions(k, plan.slices) > longest) {
+        plan = plan_product(m, n, k, true, input_gradient, longest);
+    }
+    return plan;
 }
 
 bool aligned16(const void *pointer) {
@@ -593,17 +636,19 @@ int launch_gemm_fma(const FmaGemm &g, cudaStream_t stream, int *partial_rows) {
               (!g.gelu_out || aligned16(g.gelu_out)) &&
               (!g.gelu_input || aligned16(g.gelu_input));
     p.accumulate = g.accumulate ? 1 : 0;
-    // K slices may only add into C.
     const Form form = g.a_k ? (g.b_k ? Form::InputGradient : Form::Forward)
                             : Form::WeightGradient;
-    const bool split = form == Form::WeightGradient && g.accumulate;
     if (form == Form::WeightGradient && (!g.accumulate || g.b_k)) {
         return -1;   // no caller has this form
     }
-    const FmaPlan plan = plan_product(g.m, g.n, g.k, split);
+    // K slices may only add into C.
+    const bool adds = g.accumulate && form != Form::Forward;
+    const FmaPlan plan = adds
+        ? plan_addition(g.m, g.n, g.k, form == Form::InputGradient)
+        : plan_product(g.m, g.n, g.k, false, true, LLONG_MAX);
     int slices = plan.slices;
-    p.k_per_split = ((g.k + slices - 1) / slices + 15) / 16 * 16;
-    if (split) {
+    p.k_per_split = slice_length(g.k, slices);
+    if (adds && !plan.cluster && slices > 1) {
         slices = (g.k + p.k_per_split - 1) / p.k_per_split;
         p.reduce = slices > 1 ? 1 : 0;
     }
