@@ -45,6 +45,7 @@
 #include "device_util.cuh"
 #include "gemm_tc.h"
 #include "kernels.h"
+#include "shared_limit.h"
 #include "tcgen05.cuh"
 
 #include <algorithm>
@@ -1117,16 +1118,12 @@ constexpr int smem_bytes() {
 template <int HD, int MODE>
 bool launch(const AttnMaps &maps, AttnParams params, size_t groups,
             cudaStream_t stream) {
-    static bool configured = false;
+    static SharedMemoryLimit limit;
     constexpr int bytes = smem_bytes<HD, MODE>();
     static_assert(bytes <= 227 * 1024, "shared memory");
-    if (!configured) {
-        if (cudaFuncSetAttribute(attention_tc_kernel<HD, MODE>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 bytes) != cudaSuccess) {
-            return false;
-        }
-        configured = true;
+    if (!limit.raise(reinterpret_cast<const void *>(attention_tc_kernel<HD, MODE>),
+                     bytes)) {
+        return false;
     }
     const size_t items = groups * size_t(params.row_tiles);
     if (items > size_t(INT_MAX)) {

@@ -34,6 +34,7 @@
 #include "augmentation.h"
 #include "kernels.h"
 #include "device_util.cuh"
+#include "shared_limit.h"
 
 #include <cmath>
 
@@ -500,10 +501,9 @@ void launch_augmentation(const AugmentationSettings &s,
     if (fits_shared(height * width) && batch * channels <= 0x7fffffffu) {
         const size_t bytes = 2 * ((height * width + 3) & ~size_t(3)) * sizeof(float);
         if (bytes > 40 * 1024) {
-            static const cudaError_t configured = cudaFuncSetAttribute(
-                augmentation_plane_kernel,
-                cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPlaneBytes));
-            if (configured != cudaSuccess) {
+            static SharedMemoryLimit limit;
+            if (!limit.raise(reinterpret_cast<const void *>(augmentation_plane_kernel),
+                             int(kPlaneBytes))) {
                 return;   // reported by the caller's error check
             }
         }

@@ -32,6 +32,7 @@
 #include "gemm.h"
 #include "kernels.h"
 #include "device_util.cuh"
+#include "shared_limit.h"
 
 #include <algorithm>
 #include <climits>
@@ -474,10 +475,9 @@ cudaError_t launch_form(const FmaParams &p, int slices, cudaStream_t stream) {
     constexpr size_t kBytes = kRing > kPartial ? kRing : kPartial;
     const auto kernel = fma_kernel<TM, TN, RM, RN, KB, CTAS, A_K, B_K, CLUSTER>;
     if (kBytes > 40 * 1024) {   // (some static shared memory comes on top)
-        static const cudaError_t configured = cudaFuncSetAttribute(
-            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBytes));
-        if (configured != cudaSuccess) {
-            return configured;
+        static SharedMemoryLimit limit;
+        if (!limit.raise(reinterpret_cast<const void *>(kernel), int(kBytes))) {
+            return cudaErrorInvalidConfiguration;
         }
     }
     const dim3 grid((p.m + TM - 1) / TM, (p.n + TN - 1) / TN, slices);

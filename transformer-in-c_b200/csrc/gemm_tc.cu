@@ -35,6 +35,7 @@
 #include "gemm_tc.h"
 #include "kernels.h"
 #include "device_util.cuh"
+#include "shared_limit.h"
 #include "tcgen05.cuh"
 
 #include <cuda.h>
@@ -791,31 +792,24 @@ int launch_gemm_tc(const TcGemm &g, cudaStream_t stream, int *partial_rows) {
     if (!gemm_tc_supported(g)) {
         return -1;
     }
-    static bool configured = false;
-    if (!configured) {
-        const void *kernels[] = {
-            reinterpret_cast<const void *>(gemm_tc_kernel<128, 32, 0>),
-            reinterpret_cast<const void *>(gemm_tc_kernel<128, 32, kSecondGelu>),
-            reinterpret_cast<const void *>(gemm_tc_kernel<128, 32, kGeluSlope>),
-            reinterpret_cast<const void *>(gemm_tc_kernel<128, 64, 0>),
-            reinterpret_cast<const void *>(gemm_tc_kernel<128, 64, kSecondGelu>),
-            reinterpret_cast<const void *>(gemm_tc_kernel<128, 64, kGeluSlope>),
-            reinterpret_cast<const void *>(gemm_tc_kernel<128, 128, 0>),
-            reinterpret_cast<const void *>(gemm_tc_kernel<128, 128, kSecondGelu>),
-            reinterpret_cast<const void *>(gemm_tc_kernel<128, 128, kSecondResidual>),
-            reinterpret_cast<const void *>(gemm_tc_kernel<128, 128, kGeluSlope>),
-            reinterpret_cast<const void *>(gemm_tc_kernel<128, 256, 0>),
-            reinterpret_cast<const void *>(gemm_tc_kernel<128, 256, kSecondGelu>),
-            reinterpret_cast<const void *>(gemm_tc_kernel<256, 256, 0>),
-            reinterpret_cast<const void *>(gemm_tc_kernel<256, 256, kSecondGelu>)};
-        for (const void *kernel : kernels) {
-            if (cudaFuncSetAttribute(kernel,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     kSmemLimit) != cudaSuccess) {
-                return -1;
-            }
-        }
-        configured = true;
+    static SharedMemoryLimit limit;
+    static const void *const kernels[] = {
+        reinterpret_cast<const void *>(gemm_tc_kernel<128, 32, 0>),
+        reinterpret_cast<const void *>(gemm_tc_kernel<128, 32, kSecondGelu>),
+        reinterpret_cast<const void *>(gemm_tc_kernel<128, 32, kGeluSlope>),
+        reinterpret_cast<const void *>(gemm_tc_kernel<128, 64, 0>),
+        reinterpret_cast<const void *>(gemm_tc_kernel<128, 64, kSecondGelu>),
+        reinterpret_cast<const void *>(gemm_tc_kernel<128, 64, kGeluSlope>),
+        reinterpret_cast<const void *>(gemm_tc_kernel<128, 128, 0>),
+        reinterpret_cast<const void *>(gemm_tc_kernel<128, 128, kSecondGelu>),
+        reinterpret_cast<const void *>(gemm_tc_kernel<128, 128, kSecondResidual>),
+        reinterpret_cast<const void *>(gemm_tc_kernel<128, 128, kGeluSlope>),
+        reinterpret_cast<const void *>(gemm_tc_kernel<128, 256, 0>),
+        reinterpret_cast<const void *>(gemm_tc_kernel<128, 256, kSecondGelu>),
+        reinterpret_cast<const void *>(gemm_tc_kernel<256, 256, 0>),
+        reinterpret_cast<const void *>(gemm_tc_kernel<256, 256, kSecondGelu>)};
+    if (!limit.raise(kernels, int(sizeof(kernels) / sizeof(kernels[0])), kSmemLimit)) {
+        return -1;
     }
     // Wide tiles where the product is compute-bound: deep reductions, one
     // output (or the GELU pair), a multiple of 128 columns.
