@@ -1,0 +1,48 @@
+// The host side of the augmentation's launches, with the runtime's calls that would
+// reach a device replaced: nothing here touches a GPU, present or not.
+#include "augmentation.h"
+
+#include <cstdio>
+
+static int launches = 0;
+
+extern "C" {
+cudaError_t cudaGetDevice(int *device) {
+    *device = 0;
+    return cudaSuccess;
+}
+cudaError_t cudaFuncSetAttribute(const void *, cudaFuncAttribute, int) {
+    return cudaSuccess;
+}
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *, const void *, void **) {
+    ++launches;
+    return cudaSuccess;
+}
+cudaError_t cudaLaunchKernel(const void *, dim3, dim3, void **, size_t, cudaStream_t) {
+    ++launches;
+    return cudaSuccess;
+}
+}
+
+namespace vitb200 {
+unsigned long long g_kernel_launches = 0;
+}
+
+#define CHECK(condition)                                              \
+    if (!(condition)) {                                               \
+        printf("line %d: %s\n", __LINE__, #condition);                \
+        return 1;                                                     \
+    }
+
+int main() {
+    using namespace vitb200;
+    // Scratch for every batch that does not go plane by plane, one with more planes
+    // than a grid has blocks among them.
+    CHECK(augmentation_scratch_bytes(2048, 3, 28, 28) == 0);
+    CHECK(augmentation_scratch_bytes(2, 1, 160, 160) == 0);
+    CHECK(augmentation_scratch_bytes(2, 1, 161, 160) > 0);
+    CHECK(augmentation_scratch_bytes(0x7fffffffu, 1, 1, 1) == 0);
+    CHECK(augmentation_scratch_bytes(0x80000000u, 1, 1, 1) > 0);
+    CHECK(augmentation_scratch_bytes(0x40000000u, 2, 1, 1) > 0);
+    return 0;
+}

@@ -423,8 +423,11 @@ namespace {
 // Two copies of a plane in shared memory.
 constexpr size_t kPlaneBytes = 200 * 1024;
 
-bool fits_shared(size_t plane) {
-    return 2 * ((plane + 3) & ~size_t(3)) * sizeof(float) <= kPlaneBytes;
+// Whether the kernel of one block per image plane takes the batch: the plane fits
+// shared memory twice, the planes a grid.
+bool block_per_plane(size_t batch, size_t channels, size_t plane) {
+    return 2 * ((plane + 3) & ~size_t(3)) * sizeof(float) <= kPlaneBytes &&
+           batch <= 0x7fffffffu / channels;
 }
 
 }  // namespace
@@ -484,7 +487,7 @@ void augmentation_plan(const AugmentationSettings &s, uint64_t *random_state,
 
 size_t augmentation_scratch_bytes(size_t batch, size_t channels, size_t height,
                                   size_t width) {
-    return fits_shared(height * width)
+    return block_per_plane(batch, channels, height * width)
         ? 0 : batch * (sizeof(AugmentationSample) + channels * sizeof(float));
 }
 
@@ -498,7 +501,7 @@ void launch_augmentation(const AugmentationSettings &s,
                                      s.noise_standard_deviation > 0.0f,
                                      s.minimum_value < s.maximum_value,
                                      s.erasing_probability > 0.0f};
-    if (fits_shared(height * width) && batch * channels <= 0x7fffffffu) {
+    if (block_per_plane(batch, channels, height * width)) {
         const size_t bytes = 2 * ((height * width + 3) & ~size_t(3)) * sizeof(float);
         if (bytes > 40 * 1024) {
             static SharedMemoryLimit limit;
