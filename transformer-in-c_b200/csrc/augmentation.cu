@@ -491,7 +491,7 @@ size_t augmentation_scratch_bytes(size_t batch, size_t channels, size_t height,
         ? 0 : batch * (sizeof(AugmentationSample) + channels * sizeof(float));
 }
 
-void launch_augmentation(const AugmentationSettings &s,
+bool launch_augmentation(const AugmentationSettings &s,
                          const AugmentationDraws *draws, const float *source,
                          float *destination, void *scratch, size_t batch,
                          size_t channels, size_t height, size_t width,
@@ -507,15 +507,18 @@ void launch_augmentation(const AugmentationSettings &s,
             static SharedMemoryLimit limit;
             if (!limit.raise(reinterpret_cast<const void *>(augmentation_plane_kernel),
                              int(kPlaneBytes))) {
-                return;   // reported by the caller's error check
+                return false;
             }
         }
         const unsigned threads = height * width <= 1024 ? 128 : 256;
-        launch_chained(augmentation_plane_kernel, dim3(unsigned(batch * channels)),
-                       dim3(threads), bytes, stream, source, destination, draws, s,
-                       steps, int(channels), int(height), int(width));
+        if (launch_chained(augmentation_plane_kernel, dim3(unsigned(batch * channels)),
+                           dim3(threads), bytes, stream, source, destination, draws, s,
+                           steps, int(channels), int(height),
+                           int(width)) != cudaSuccess) {
+            return false;
+        }
         ++g_kernel_launches;
-        return;
+        return true;
     }
     AugmentationSample *samples = static_cast<AugmentationSample *>(scratch);
     float *means = reinterpret_cast<float *>(samples + batch);
@@ -547,6 +550,7 @@ void launch_augmentation(const AugmentationSettings &s,
             int(width));
         ++g_kernel_launches;
     }
+    return cudaPeekAtLastError() == cudaSuccess;
 }
 
 void launch_augmentation_translate(const float *source, float *destination,

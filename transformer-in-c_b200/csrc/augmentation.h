@@ -64,8 +64,9 @@ size_t augmentation_scratch_bytes(size_t batch, size_t channels, size_t height,
 
 // Applies a plan.  source / destination / scratch are device pointers, draws
 // anything the device can read.  source == destination is allowed when no
-// geometric transform is configured.
-void launch_augmentation(const AugmentationSettings &settings,
+// geometric transform is configured.  False when a kernel could not be launched; the
+// destination's contents are then undefined.
+bool launch_augmentation(const AugmentationSettings &settings,
                          const AugmentationDraws *draws, const float *source,
                          float *destination, void *scratch, size_t batch,
                          size_t channels, size_t height, size_t width,

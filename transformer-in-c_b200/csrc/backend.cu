@@ -2737,8 +2737,8 @@ extern "C" int vitb200_data_augmentation_apply(
               "cudaHostGetDevicePointer");
         slot.capacity = batch;
     }
-    augmentation_plan(*settings, random_state, batch, channels, height, width,
-                      slot.host);
+    uint64_t state = *random_state;
+    augmentation_plan(*settings, &state, batch, channels, height, width, slot.host);
     const size_t count = batch * channels * height * width;
     const size_t scratch_bytes =
         augmentation_scratch_bytes(batch, channels, height, width);
@@ -2760,11 +2760,16 @@ extern "C" int vitb200_data_augmentation_apply(
         in = augment_input(backend, source, count);
         out = augment_output(backend, destination, count, &staged);
     }
+    bool launched = false;
     {
         OpScope scope(backend, "data_augmentation", 8.0 * double(count), 0.0);
-        launch_augmentation(*settings, slot.device, in, out, work, batch, channels,
-                            height, width, backend->stream);
+        launched = launch_augmentation(*settings, slot.device, in, out, work, batch,
+                                       channels, height, width, backend->stream);
     }
+    if (!launched) {
+        return -1;
+    }
+    *random_state = state;
     check(cudaEventRecord(slot.read, backend->stream), "cudaEventRecord");
     augment_finish(backend, destination, out, count, staged);
     return 0;
