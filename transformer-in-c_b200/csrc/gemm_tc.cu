@@ -765,6 +765,60 @@ int *status_word() {
     return word;
 }
 
+using TcKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap,
+                          const CUtensorMap, const TcParams);
+
+// A tile with the kernels built for it, by epilogue.  Boxes of the tensor maps, bytes of
+// a stage, ring depth and grid all follow m and n, and a kernel that is handed another
+// tile's would write out of range: so kernels are named here, beside their extents,
+// and nowhere else.
+struct TcTile {
+    int m, n, threads;
+    TcKernel plain, second_gelu, second_residual, gelu_slope;   // null: not built
+
+    TcKernel kernel(int second) const {
+        return second == kSecondGelu       ? second_gelu
+               : second == kSecondResidual ? second_residual
+               : second == kGeluSlope      ? gelu_slope
+                                           : plain;
+    }
+};
+
+template <int M, int N>
+constexpr TcTile make_tile() {
+    TcTile tile = {M, N, M == 2 * kTileM ? kThreadsTall : kThreads,
+                   gemm_tc_kernel<M, N, 0>, gemm_tc_kernel<M, N, kSecondGelu>,
+                   nullptr, nullptr};
+    if constexpr (M == kTileM && N <= kTileN) {
+        tile.gelu_slope = gemm_tc_kernel<M, N, kGeluSlope>;
+    }
+    if constexpr (M == kTileM && N == kTileN) {
+        tile.second_residual = gemm_tc_kernel<M, N, kSecondResidual>;
+    }
+    return tile;
+}
+
+enum { kNarrow32, kNarrow64, kSquare, kWide, kTall, kTcTileCount };
+const TcTile kTcTiles[kTcTileCount] = {
+    make_tile<kTileM, 32>(), make_tile<kTileM, 64>(), make_tile<kTileM, kTileN>(),
+    make_tile<kTileM, 256>(), make_tile<2 * kTileM, 256>()};
+
+// Lets every kernel use the whole of an SM's shared memory.
+bool raise_limits() {
+    static SharedMemoryLimit limit;
+    const void *kernels[4 * kTcTileCount];
+    int count = 0;
+    for (const TcTile &tile : kTcTiles) {
+        for (TcKernel kernel : {tile.plain, tile.second_gelu, tile.second_residual,
+                                tile.gelu_slope}) {
+            if (kernel) {
+                kernels[count++] = reinterpret_cast<const void *>(kernel);
+            }
+        }
+    }
+    return limit.raise(kernels, count, kSmemLimit);
+}
+
 }  // namespace
 
 bool gemm_tc_supported(const TcGemm &g) {
@@ -792,23 +846,7 @@ int launch_gemm_tc(const TcGemm &g, cudaStream_t stream, int *partial_rows) {
     if (!gemm_tc_supported(g)) {
         return -1;
     }
-    static SharedMemoryLimit limit;
-    static const void *const kernels[] = {
-        reinterpret_cast<const void *>(gemm_tc_kernel<128, 32, 0>),
-        reinterpret_cast<const void *>(gemm_tc_kernel<128, 32, kSecondGelu>),
-        reinterpret_cast<const void *>(gemm_tc_kernel<128, 32, kGeluSlope>),
-        reinterpret_cast<const void *>(gemm_tc_kernel<128, 64, 0>),
-        reinterpret_cast<const void *>(gemm_tc_kernel<128, 64, kSecondGelu>),
-        reinterpret_cast<const void *>(gemm_tc_kernel<128, 64, kGeluSlope>),
-        reinterpret_cast<const void *>(gemm_tc_kernel<128, 128, 0>),
-        reinterpret_cast<const void *>(gemm_tc_kernel<128, 128, kSecondGelu>),
-        reinterpret_cast<const void *>(gemm_tc_kernel<128, 128, kSecondResidual>),
-        reinterpret_cast<const void *>(gemm_tc_kernel<128, 128, kGeluSlope>),
-        reinterpret_cast<const void *>(gemm_tc_kernel<128, 256, 0>),
-        reinterpret_cast<const void *>(gemm_tc_kernel<128, 256, kSecondGelu>),
-        reinterpret_cast<const void *>(gemm_tc_kernel<256, 256, 0>),
-        reinterpret_cast<const void *>(gemm_tc_kernel<256, 256, kSecondGelu>)};
-    if (!limit.raise(kernels, int(sizeof(kernels) / sizeof(kernels[0])), kSmemLimit)) {
+    if (!raise_limits()) {
         return -1;
     }
     // Wide tiles where the product is compute-bound: deep reductions, one
@@ -865,24 +903,30 @@ int launch_gemm_tc(const TcGemm &g, cudaStream_t stream, int *partial_rows) {
     // (13 tiles before, 52 now), [1600,128]x[128,512] 7.6 -> 5.6 us, with GELU
     // 10.4 -> 7.8; a step of batch 32 762 -> 668 us, of 117 colour images
     // 559 -> 530 us.  With one tile per SM as the limit these were 673 and 542.
-    int narrow = 0;
+    int narrow = -1;
     if (!g.residual && !forced_tile && !forced_tile_m) {
         const long long row_tiles = (g.m + kTileM - 1) / kTileM;
         // (The slices of a split reduction, four blocks each at least.)
         const long long slices =
             g.accumulate ? std::max(1, (g.k + kBlockK - 1) / kBlockK / 4) : 1;
-        for (int width = 32; width < kTileN && !narrow; width *= 2) {
-            if (row_tiles * ((g.n + width - 1) / width) * slices <=
-                2 * (long long)device_sm_count()) {
-                narrow = width;
+        for (int candidate : {kNarrow32, kNarrow64}) {
+            const int width = kTcTiles[candidate].n;
+            if (narrow < 0 && row_tiles * ((g.n + width - 1) / width) * slices <=
+                                  2 * (long long)device_sm_count()) {
+                narrow = candidate;
             }
         }
     }
-    if (narrow) {
-        wide = tall = false;
+    // From here on only the tile counts.
+    const TcTile &tile =
+        kTcTiles[narrow >= 0 ? narrow : (tall ? kTall : (wide ? kWide : kSquare))];
+    const int tile_m = tile.m, tile_n = tile.n;
+    const int second = g.d2 ? (g.residual ? kSecondResidual : kSecondGelu)
+                            : (g.gelu_input ? kGeluSlope : 0);
+    const TcKernel kernel = tile.kernel(second);
+    if (!kernel) {
+        return -1;
     }
-    const int tile_n = narrow ? narrow : (wide ? 256 : kTileN);
-    const int tile_m = tall ? 2 * kTileM : kTileM;
     CUtensorMap map_a, map_b, map_d;
     // K-major operand: rows = output index, inner = reduction index.
     // MN-major operand: rows = reduction index, inner = output index.
@@ -942,11 +986,11 @@ int launch_gemm_tc(const TcGemm &g, cudaStream_t stream, int *partial_rows) {
     if (forced_ctas > 0) {
         ctas_per_sm = forced_ctas;
     }
-    if (wide) {
+    if (tile_n > kTileN) {
         // One CTA per SM (it owns all of tensor memory): four 48 KiB stages
         // and double-buffered staging, 224 KiB.
         ctas_per_sm = 1;
-        p.stages = tall ? 3 : 4;   // 64 KiB stages when the tile is tall
+        p.stages = tile_m > kTileM ? 3 : 4;   // 64 KiB stages when the tile is tall
         staging_bytes = 2 * kOperandBytes;
     }
     if (forced_staging == 1 && !(g.d2 && g.residual)) {
@@ -954,19 +998,20 @@ int launch_gemm_tc(const TcGemm &g, cudaStream_t stream, int *partial_rows) {
     } else if (forced_staging == 2 || (forced_stages > 0 && forced_staging == 0)) {
         staging_bytes = 2 * kOperandBytes;
     }
-    const bool spread = narrow && (long long)tiles <= (long long)device_sm_count();
-    if (narrow && forced_stages == 0) {
+    const bool narrowed = tile_n < kTileN;
+    const bool spread = narrowed && (long long)tiles <= (long long)device_sm_count();
+    if (narrowed && forced_stages == 0) {
         // The ring as deep as the reduction, where a CTA has the SM to itself.
         const int depth = spread && !g.accumulate ? kMaxStages : 4;
         p.stages = std::max(2, std::min(depth, p.k_blocks));
     }
     if (g.gelu_input) {
         staging_bytes = 2 * kOperandBytes;   // its epilogue pipeline needs both blocks
-        if (p.stages > 2 && ctas_per_sm > 1 && !narrow) {
+        if (p.stages > 2 && ctas_per_sm > 1 && !narrowed) {
             p.stages = 2;
         }
     }
-    if (narrow) {
+    if (narrowed) {
         // What fits beside the staging blocks, for one or for two CTAs per SM.
         const int room = (spread ? kSmemLimit : kSmemLimit / 2) - staging_bytes -
                          kBarrierBytes;
@@ -1005,8 +1050,6 @@ int launch_gemm_tc(const TcGemm &g, cudaStream_t stream, int *partial_rows) {
     p.b_mn_major = g.b_mn_major ? 1 : 0;
     p.reduce_add = g.accumulate ? 1 : 0;
     p.bias = g.bias;
-    const int second = g.d2 ? (g.residual ? kSecondResidual : kSecondGelu)
-                            : (g.gelu_input ? kGeluSlope : 0);
     p.column_partials = g.column_partials;
     p.residual = g.residual;
     p.residual_pitch = g.ld_residual;
@@ -1027,36 +1070,11 @@ int launch_gemm_tc(const TcGemm &g, cudaStream_t stream, int *partial_rows) {
     if (g.column_partials && partial_rows) {
         *partial_rows = int(grid);
     }
-    auto launch = [&](auto kernel, int threads) {
-        launch_chained(kernel, grid, threads, smem_bytes, stream, map_a, map_b,
-                       map_d, map_d2, p);
-    };
-    if (tall && second == kSecondGelu) {
-        launch(gemm_tc_kernel<256, 256, kSecondGelu>, kThreadsTall);
-    } else if (tall) {
-        launch(gemm_tc_kernel<256, 256, 0>, kThreadsTall);
-    } else if (wide && second == kSecondGelu) {
-        launch(gemm_tc_kernel<128, 256, kSecondGelu>, kThreads);
-    } else if (wide) {
-        launch(gemm_tc_kernel<128, 256, 0>, kThreads);
-    } else if (second == kSecondResidual) {
-        launch(gemm_tc_kernel<128, 128, kSecondResidual>, kThreads);
-    } else if (second == kSecondGelu) {
-        launch(narrow == 32   ? gemm_tc_kernel<128, 32, kSecondGelu>
-               : narrow == 64 ? gemm_tc_kernel<128, 64, kSecondGelu>
-                              : gemm_tc_kernel<128, 128, kSecondGelu>, kThreads);
-    } else if (second == kGeluSlope) {
-        launch(narrow == 32   ? gemm_tc_kernel<128, 32, kGeluSlope>
-               : narrow == 64 ? gemm_tc_kernel<128, 64, kGeluSlope>
-                              : gemm_tc_kernel<128, 128, kGeluSlope>, kThreads);
-    } else {
-        launch(narrow == 32   ? gemm_tc_kernel<128, 32, 0>
-               : narrow == 64 ? gemm_tc_kernel<128, 64, 0>
-                              : gemm_tc_kernel<128, 128, 0>, kThreads);
-    }
+    launch_chained(kernel, grid, tile.threads, smem_bytes, stream, map_a, map_b, map_d,
+                   map_d2, p);
     ++g_kernel_launches;
     ++g_tc_products;
-    if (wide) {
+    if (tile_n > kTileN) {
         ++g_tc_wide_products;
     }
     return 0;
