@@ -59,9 +59,35 @@ def augmentation_errors(case):
             "pixel": float(np.abs(out - expected).max())}
 
 
+def shared_allocations(case):
+    """Weights at the front of an allocation that holds more: a step updates them like
+    weights with one of their own and leaves the rest alone.  Returns how many of
+    either differ."""
+    rest = 1000
+    states = [cases.prepare(case, 3) for _ in range(2)]
+    for name, p in states[1].model.parameters.items():
+        count = p.rows * p.cols
+        memory = cases._Memory(count + rest)
+        memory.array()[:count] = p.data.array()
+        memory.array()[count:] = np.arange(rest)
+        p.data, p.struct.data = memory, memory.address
+    for _ in range(3):
+        for state in states:
+            state.train()
+    plain, shared = (state.model.parameters for state in states)
+    found = {"values": 0, "rest": 0}
+    for name, p in plain.items():
+        count = p.rows * p.cols
+        found["values"] += int((shared[name].data.array()[:count] != p.data.array()).sum())
+        found["rest"] += int((shared[name].data.array()[count:] != np.arange(rest)).sum())
+    return found
+
+
 def errors(case):
     if case["kind"] == "augment":
         return augmentation_errors(case)
+    if case.get("shared_allocations"):
+        return shared_allocations(case)
     state = cases.prepare(case, 3)
     model = state.model
     declined = state.host.backend.declined_ops()

@@ -74,6 +74,15 @@ def test_training_steps_match_the_oracle(cases, bound, loss_bound):
         assert errors.get("value", 0.0) <= 10 * bound, (case, errors)
 
 
+def test_weights_at_the_front_of_a_larger_allocation():
+    """Their update may go on in another buffer (see device_view_update), which must
+    not lose what the host keeps behind them.  (One small step after another repeats
+    bit for bit: its products have no slices that meet in memory.)"""
+    case = dict(train(2, model(1, 8, 4, 32, 4, 1, 2), precision="fp32"),
+                shared_allocations=True)
+    assert run([case]) == [{"values": 0, "rest": 0}]
+
+
 SETTINGS = dict(max_shift_pixels=2.0, max_rotation_degrees=10.0, max_scale_delta=0.1,
                 max_brightness_delta=0.05, max_contrast_delta=0.1,
                 noise_standard_deviation=0.01, erasing_probability=0.5,

@@ -2181,8 +2181,9 @@ int build_slice_table(CudaBackend *backend,
         if (with_moments) {
             // A weight that pending definitions still read (the skipped
             // gradients of op_gelu_backward) is updated into another buffer.
-            slice.value = device_view_update(p->value.data, backend->stream,
-                                             &slice.value_in);
+            slice.value = device_view_update(p->value.data,
+                                             numel(&p->value) * sizeof(float),
+                                             backend->stream, &slice.value_in);
         }
         slice.grad = view(backend, p->value.grad, Access::ReadWrite);
         slice.m = with_moments ? view(backend, p->m, Access::ReadWrite) : nullptr;

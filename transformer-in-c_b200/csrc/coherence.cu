@@ -1091,10 +1091,10 @@ float *device_view_accumulate_based(const void *host_pointer,
     return own;
 }
 
-float *device_view_update(const void *host_pointer, cudaStream_t stream,
+float *device_view_update(const void *host_pointer, size_t bytes, cudaStream_t stream,
                           const float **current) {
     Region *region = host_pointer ? find_base(host_pointer) : nullptr;
-    if (!region || !region->feeds || !region->device || region->lazy ||
+    if (!region || region->bytes > bytes || !region->feeds || !region->device || region->lazy ||
         region->zero_pending || region->owner == Owner::Host) {
         float *own = device_view(host_pointer, Access::ReadWrite, stream);
         *current = own;
@@ -1102,7 +1102,7 @@ float *device_view_update(const void *host_pointer, cudaStream_t stream,
     }
     *current = region->device;
     detach_source(*region);
-    // The contents are all rewritten, so this is an overwrite to the rest of
+    // The whole buffer is rewritten, so this is an overwrite to the rest of
     // the layer (no definition hangs on the buffer any more).
     return device_view(host_pointer, Access::Overwrite, stream);
 }

@@ -109,11 +109,12 @@ bool coherent_define_alias(const void *output_host, const void *source_host,
 // contents are a pending zero fill).  Every element must be written.
 float *device_view_accumulate_based(const void *host_pointer,
                                     cudaStream_t stream, const float **base);
-// For an update that reads every element of a buffer from *current and writes
-// it to the returned pointer.  The two are the same unless definitions that
+// For an update that reads the first `bytes` of a buffer from *current and writes
+// them to the returned pointer.  The two are the same unless definitions that
 // read the buffer are pending (a weight matrix under the optimiser): those keep
-// the old buffer then and the values go on in a fresh one, with no copy made.
-float *device_view_update(const void *host_pointer, cudaStream_t stream,
+// the old buffer then and the values go on in a fresh one, with no copy made (unless
+// the allocation holds more than `bytes`, which has to move along).
+float *device_view_update(const void *host_pointer, size_t bytes, cudaStream_t stream,
                           const float **current);
 // For an output pending under `function` with one source: copies the
 // definition's arguments out and returns the device pointer that currently
