@@ -83,7 +83,63 @@ def shared_allocations(case):
     return found
 
 
+def gelu_parameter_errors():
+    """Two products of GELU outputs, the first of which is a parameter itself: its
+    gradient is a pending definition that reads the first weights, the second weights
+    have one too, and the optimiser gets them in the order (weights, GELU output,
+    weights).  Largest error of each after the step, in learning rates."""
+    rng = np.random.default_rng(11)
+    host, n, k, m = cases._the_host(), 64, 32, 48
+    host.configure({"precision": "fp32", "deferred": False})
+    tensors = {name: cases._Tensor(*shape) for name, shape in (
+        ("h1", (n, k)), ("h2", (n, k)), ("a2", (n, k)), ("y1", (n, m)), ("y2", (n, m)))}
+    parameters = {name: cases._Parameter(*shape) for name, shape in (
+        ("w1", (k, m)), ("a1", (n, k)), ("w2", (k, m)))}
+    both = {**tensors, **parameters}
+    values = {name: rng.standard_normal((t.rows, t.cols)).astype(np.float32)
+              for name, t in both.items()}
+    for name, t in both.items():
+        t.array()[:] = values[name]
+    for p in parameters.values():
+        p.m.array()[:] = 0.0
+        p.v.array()[:] = 0.0
+        p.parameter.step = 1
+
+    def op(slot, *arguments):
+        assert host.ops[slot](host.table_context, *arguments) == 0, slot
+
+    pointer = {name: t.pointer for name, t in both.items()}
+    kept = cases._pointers(list(pointer.values()))
+    op("zero_gradients", ctypes.addressof(kept), len(kept))
+    for i in "12":
+        op("gelu", pointer["h" + i], pointer["a" + i])
+        op("gemm", pointer["a" + i], pointer["w" + i], pointer["y" + i])
+    dy = {i: rng.standard_normal((n, m)).astype(np.float32) for i in "12"}
+    for i in "12":
+        tensors["y" + i].grad.array()[:] = dy[i].ravel()
+        op("gemm_backward", pointer["a" + i], pointer["w" + i], pointer["y" + i])
+        op("gelu_backward", pointer["h" + i], pointer["a" + i])
+    table = cases._pointers([parameters[name].pointer for name in ("w1", "a1", "w2")])
+    decays = (ctypes.c_float * 3)(0.0, 0.0, 0.0)
+    op("adamw_step_parameters", ctypes.addressof(table), ctypes.addressof(decays), 3,
+       cases.LEARNING_RATE, 0.9, 0.999, 1e-8, 0.0)
+    host.synchronize()
+    found = {}
+    activated = {i: vo.gelu(values["h" + i].astype(np.float64)) for i in "12"}
+    for name, value, gradient in (
+            ("w1", values["w1"], activated["1"].T @ dy["1"]),
+            ("a1", activated["1"], dy["1"].astype(np.float64) @ values["w1"].T),
+            ("w2", values["w2"], activated["2"].T @ dy["2"])):
+        want, _, _ = vo.adamw_update(value.astype(np.float64), gradient, 0.0 * gradient,
+                                     0.0 * gradient, 1, cases.LEARNING_RATE, 0.0)
+        found[name] = float(np.abs(parameters[name].array() - want).max()
+                            / cases.LEARNING_RATE)
+    return found
+
+
 def errors(case):
+    if case["kind"] == "gelu_parameter":
+        return gelu_parameter_errors()
     if case["kind"] == "augment":
         return augmentation_errors(case)
     if case.get("shared_allocations"):

@@ -83,6 +83,15 @@ def test_weights_at_the_front_of_a_larger_allocation():
     assert run([case]) == [{"values": 0, "rest": 0}]
 
 
+def test_update_of_a_parameter_with_a_pending_gradient():
+    """Computing it gives a buffer back that another weight of the same update is still
+    read from.  A first step moves every value by the learning rate, in its gradient's
+    sign; values of about one are rounded to 6e-8, 6e-5 of that."""
+    (found,) = run([dict(kind="gelu_parameter")])
+    assert found.keys() == {"w1", "a1", "w2"}
+    assert max(found.values()) <= 1e-3, found
+
+
 SETTINGS = dict(max_shift_pixels=2.0, max_rotation_degrees=10.0, max_scale_delta=0.1,
                 max_brightness_delta=0.05, max_contrast_delta=0.1,
                 noise_standard_deviation=0.01, erasing_probability=0.5,

@@ -2168,6 +2168,19 @@ int build_slice_table(CudaBackend *backend,
         block_elements *= 2;
     }
     slices->resize(count);
+    // Everything that computes a pending definition first: its sources' old buffers
+    // may go back to the pool then, and one of them could be where a weight below is
+    // read from and where the next one's fresh buffer comes from.
+    for (size_t i = 0; i < count; ++i) {
+        vitb200_parameter *p = parameters[i];
+        ParameterSlice &slice = (*slices)[i];
+        slice.grad = view(backend, p->value.grad, Access::ReadWrite);
+        slice.m = with_moments ? view(backend, p->m, Access::ReadWrite) : nullptr;
+        slice.v = with_moments ? view(backend, p->v, Access::ReadWrite) : nullptr;
+        if (with_moments && coherent_is_lazy(p->value.data)) {
+            view(backend, p->value.data, Access::ReadWrite);
+        }
+    }
     unsigned long long blocks = 0;
     // The host has advanced the steps together (reference src/ops.c:1140-1142),
     // so the corrections rarely differ from one parameter to the next.
@@ -2185,9 +2198,6 @@ int build_slice_table(CudaBackend *backend,
                                              numel(&p->value) * sizeof(float),
                                              backend->stream, &slice.value_in);
         }
-        slice.grad = view(backend, p->value.grad, Access::ReadWrite);
-        slice.m = with_moments ? view(backend, p->m, Access::ReadWrite) : nullptr;
-        slice.v = with_moments ? view(backend, p->v, Access::ReadWrite) : nullptr;
         slice.count = numel(&p->value);
         slice.first_block = unsigned(blocks);
         slice.weight_decay = weight_decays ? weight_decays[i] : 0.0f;
