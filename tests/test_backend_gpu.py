@@ -611,8 +611,9 @@ def test_unread_tensors_are_not_computed_but_reads_see_them(vit_host_module,
     # (views of the projected / merged matrices); and the same five gradients
     # less P's, which nobody produces.
     # On top of those, the gradients that residual_backward and
-    # accumulate_gradient would merely copy (four per block) are aliases.
-    per_block = 1 + 4 + 4 + 4
+    # accumulate_gradient would merely copy (four per block) are aliases, and the
+    # gradient of the GELU output is not stored.
+    per_block = 1 + 4 + 4 + 4 + 1
     assert after["lazy_defined"] - before["lazy_defined"] == 2 * per_block * layers
     assert after["lazy_materialised"] == before["lazy_materialised"]
     # Every definition of step 1 has been dropped (overwritten, re-zeroed or
