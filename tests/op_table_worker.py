@@ -34,6 +34,11 @@ def oracle_name(name):
     return f"{layer}.{BLOCK[head]}" + (f"_{tail}" if tail else "")
 
 
+def larger(worst, error):
+    """The larger of two errors; not a number if either is (max would drop it)."""
+    return float(np.maximum(worst, error))
+
+
 def batch_of(state, case, k):
     if state.resident is None:
         labels = state.labels[k].astype(int) if case["kind"] == "train" else None
@@ -137,13 +142,86 @@ def gelu_parameter_errors():
     return found
 
 
+def slope_product_errors(case):
+    """A product behind a GELU and a bias, backward, in FP32: the gradient before the
+    GELU and its column sums, the weights' gradient and the skipped gradient, each
+    against its largest entry."""
+    rng = np.random.default_rng(case["m"])
+    host, m, k, n = cases._the_host(), case["m"], case["k"], case["n"]
+    host.configure({"precision": "fp32", "deferred": False})
+    tensors = {name: cases._Tensor(*shape) for name, shape in (
+        ("hidden", (m, k)), ("bias", (1, k)), ("activated", (m, k)), ("w", (k, n)),
+        ("y", (m, n)))}
+    pointer = {name: t.pointer for name, t in tensors.items()}
+
+    def op(slot, *arguments):
+        assert host.ops[slot](host.table_context, *arguments) == 0, slot
+
+    kept = cases._pointers(list(pointer.values()))
+    op("zero_gradients", ctypes.addressof(kept), len(kept))
+    values = {name: rng.standard_normal((t.rows, t.cols)).astype(np.float32)
+              for name, t in tensors.items()}
+    for name in ("hidden", "w"):
+        tensors[name].array()[:] = values[name]
+    op("gelu", pointer["hidden"], pointer["activated"])
+    op("gemm", pointer["activated"], pointer["w"], pointer["y"])
+    tensors["y"].grad.array()[:] = values["y"].ravel()
+    fused = host.backend.fusion_counters()["epilogues"]
+    op("gemm_backward", pointer["activated"], pointer["w"], pointer["y"])
+    op("gelu_backward", pointer["hidden"], pointer["activated"])
+    op("bias_add_backward", pointer["hidden"], pointer["bias"])
+    host.synchronize()
+    found = {"fused": host.backend.fusion_counters()["epilogues"] - fused}
+    hidden, w, dy = (values[name].astype(np.float64) for name in ("hidden", "w", "y"))
+    skipped = dy @ w.T
+    before = vo.gelu_backward(hidden, skipped)
+    for name, want in (("hidden", before), ("bias", before.sum(axis=0, keepdims=True)),
+                       ("w", vo.gelu(hidden).T @ dy), ("activated", skipped)):
+        got = tensors[name].grad.array().reshape(want.shape)
+        found[name] = float(np.abs(got - want).max() / np.abs(want).max())
+    return found
+
+
+def skipped_gradients(case):
+    """The gradients of the GELU outputs, which no kernel stores, read after the
+    optimiser has moved the weights they are defined by: largest error against
+    dY W^T with the weights of before the step, and against those of after it; and how
+    many definitions a block and step make, and the reads compute."""
+    state = cases.prepare(case, 3)
+    tensors, parameters = state.model.tensors, state.model.parameters
+    counters = state.host.backend.elision_counters
+    state.train()   # (the first step uploads)
+    found = {"before": 0.0, "after": 0.0}
+    old = {name: np.array(p.array(), np.float64) for name, p in parameters.items()}
+    start = counters()
+    state.train()
+    end = counters()
+    found["defined"] = (end["lazy_defined"] - start["lazy_defined"]) / case["layers"]
+    for layer in range(case["layers"]):
+        activated, branch = (
+            tensors["%d.%s" % (layer, name)] for name in ("activated", "branch2"))
+        dy = branch.grad.array().astype(np.float64).reshape(branch.rows, branch.cols)
+        start = counters()
+        dx = activated.grad.array().astype(np.float64).reshape(activated.rows, -1)
+        found["computed"] = counters()["lazy_materialised"] - start["lazy_materialised"]
+        name = "%d.fc2" % layer
+        for key, w in (("before", old[name]), ("after", parameters[name].array())):
+            want = dy @ w.astype(np.float64).T
+            found[key] = larger(found[key], np.abs(dx - want).max() / np.abs(want).max())
+    return found
+
+
 def errors(case):
+    if case["kind"] == "slope_product":
+        return slope_product_errors(case)
     if case["kind"] == "gelu_parameter":
         return gelu_parameter_errors()
     if case["kind"] == "augment":
         return augmentation_errors(case)
     if case.get("shared_allocations"):
         return shared_allocations(case)
+    if case.get("skipped_gradients"):
+        return skipped_gradients(case)
     state = cases.prepare(case, 3)
     model = state.model
     declined = state.host.backend.declined_ops()
@@ -173,7 +251,7 @@ def errors(case):
             grads[name] = grads.get(name, 0.0) + value / micro
     scale, _ = vo.clip_scale(list(grads.values()), cases.CLIP_NORM)
     got = cases.run(state)
-    worst = {"loss": abs(got["loss"] - float(np.mean(losses))), "gradient": 0.0,
+    worst = {"loss": float(abs(got["loss"] - np.mean(losses))), "gradient": 0.0,
              "moment": 0.0, "value": 0.0}
     d = case["width"]
     for name, p in model.parameters.items():
@@ -196,7 +274,7 @@ def errors(case):
         for key, error in (("gradient", np.abs(gradient - want).max() / largest),
                            ("moment", moment.max() / np.abs(v).max()),
                            ("value", change.max() / cases.LEARNING_RATE)):
-            worst[key] = max(worst[key], float(error))
+            worst[key] = larger(worst[key], error)
     worst["declined"] = state.host.backend.declined_ops() - declined
     return worst
 

@@ -45,6 +45,10 @@ FP32 = [
     train(5, model(1, 28, 7, 40, 5, 1, 13), micro=2, deferred=True),
     train(40, model(1, 28, 4, 128, 8, 1, 11), precision="fp32"),
     train(300, model(1, 16, 4, 64, 4, 1, 10), precision="fp32", deferred=True),
+    # More rows of column sums in the slope product than there is room for: shared.
+    train(400, model(1, 28, 4, 64, 4, 1, 10), precision="fp32"),
+    # More parameters (212) than the optimiser's kernels take as arguments.
+    train(2, model(1, 8, 4, 32, 4, 17, 3)),
 ]
 TF32 = [
     train(32, model(1, 28, 4, 128, 8, 2, 11)),
@@ -66,12 +70,17 @@ def test_training_steps_match_the_oracle(cases, bound, loss_bound):
     found = run(cases)
     assert len(found) == len(cases)
     for case, errors in zip(cases, found):
-        assert errors.get("declined", 0) == 0, (case, errors)
-        assert errors.get("logits", 0.0) <= bound, (case, errors)
-        assert errors.get("loss", 0.0) <= loss_bound, (case, errors)
-        assert errors.get("gradient", 0.0) <= bound, (case, errors)
-        assert errors.get("moment", 0.0) <= 2 * bound, (case, errors)
-        assert errors.get("value", 0.0) <= 10 * bound, (case, errors)
+        assert within(errors, bound, loss_bound), (case, errors)
+
+
+def within(errors, bound, loss_bound):
+    """Not a number is within nothing."""
+    return (errors.get("declined", 0) == 0 and
+            errors.get("logits", 0.0) <= bound and
+            errors.get("loss", 0.0) <= loss_bound and
+            errors.get("gradient", 0.0) <= bound and
+            errors.get("moment", 0.0) <= 2 * bound and
+            errors.get("value", 0.0) <= 10 * bound)
 
 
 def test_weights_at_the_front_of_a_larger_allocation():
@@ -89,7 +98,36 @@ def test_update_of_a_parameter_with_a_pending_gradient():
     sign; values of about one are rounded to 6e-8, 6e-5 of that."""
     (found,) = run([dict(kind="gelu_parameter")])
     assert found.keys() == {"w1", "a1", "w2"}
-    assert max(found.values()) <= 1e-3, found
+    assert all(error <= 1e-3 for error in found.values()), found
+
+
+def test_slope_products_on_the_fma_tiles():
+    """One row, rows that no vector access fits, slices in a cluster, ragged tiles, and
+    more rows of column sums than there is room for (313 and 704 for 296).  FP32 sums of
+    n terms, of m for the weights and the bias: 2e-5 of the largest entry."""
+    cases = [dict(kind="slope_product", m=m, k=k, n=n) for m, k, n in (
+        (1, 5, 3), (50, 512, 128), (50, 33, 515), (300, 257, 66), (4329, 33, 7),
+        (4329, 130, 72), (20000, 128, 512), (45000, 64, 30))]
+    found = run(cases)
+    assert len(found) == len(cases)
+    for case, errors in zip(cases, found):
+        assert errors.pop("fused") == 1, (case, errors)
+        assert all(error <= 2e-5 for error in errors.values()), (case, errors)
+
+
+def test_skipped_gradients_are_those_of_the_weights_before_the_step():
+    """Bounds as for the products (FP32 2e-5, TF32 2e-3 of the largest entry); a step
+    moves the weights by about a hundredth of themselves.  Definitions of a block and
+    step: the probabilities, four head views forward and four backward, four aliases
+    and the skipped gradient; the read computes the latter alone."""
+    shape = model(1, 28, 4, 64, 4, 2, 11)
+    cases = [dict(train(4, shape, precision="fp32"), skipped_gradients=True),
+             dict(train(32, shape), skipped_gradients=True)]
+    found = run(cases)
+    for errors, bound in zip(found, (2e-5, 2e-3)):
+        assert errors["before"] <= bound < errors["after"] / 2, errors
+        assert errors["defined"] == 14 and errors["computed"] == 1, errors
+    assert len(found) == len(cases)
 
 
 SETTINGS = dict(max_shift_pixels=2.0, max_rotation_degrees=10.0, max_scale_delta=0.1,
@@ -114,6 +152,8 @@ def test_augmentation_in_one_kernel_and_in_three():
                  (3, 2, 1, 1, SETTINGS), (9, 1, 33, 32, WITHOUT_NOISE),
                  (4, 3, 12, 31, ONLY_NOISE), (2, 1, 160, 160, SETTINGS),
                  (2, 1, 161, 160, SETTINGS))]
-    for case, errors in zip(cases, run(cases)):
+    found = run(cases)
+    assert len(found) == len(cases)
+    for case, errors in zip(cases, found):
         assert errors["status"] == 0 and errors["stream"] == 0, case
         assert errors["pixel"] <= 2.1e-6, (case, errors)
