@@ -328,7 +328,8 @@ attention_small_backward_kernel(
     HeadLayout grad_layout) {
     extern __shared__ __align__(16) float shared[];
     constexpr int kPitch = kTilePitch<HD>;
-    constexpr bool kTwoTiles = HD < 64 && LANES > 1;   // as two_score_tiles()   // P and dS side by side
+    constexpr bool kTwoTiles = HD < 64 && LANES > 1;   // P and dS side by side,
+                                                       // as two_score_tiles()
     const int pitch = seq | 1;
     float *q_tile = shared;
     float *k_tile = q_tile + seq * kPitch;

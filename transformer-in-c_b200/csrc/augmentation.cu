@@ -5,11 +5,11 @@
 // by a constant per draw, so draw number k is mix(state + (k + 1) * step): a
 // pure function of the start state.  The order of the draws is fixed except
 // for random erasing, which takes four more draws only when its first draw
-// says "erase".  A host pass over the batch (a dozen integer mixes per sample)
-// therefore knows where each sample's draws start; after that every sample is
-// independent.  The host keeps only what cannot move: the walk along the stream
-// (one mix per sample, for the erasing decision) and the rotation's cosine and
-// sine, which have to come from the same libm as the reference's.
+// says "erase".  A host pass over the batch therefore knows where each sample's
+// draws start; after that every sample is independent.  The host keeps only what
+// cannot move: the walk along the stream (one mix per sample, for the erasing
+// decision) and the rotation's angle, cosine and sine (a second mix), which have to
+// come from the same libm as the reference's.
 //
 // Images whose plane fits shared memory twice (up to 160 x 160) take one kernel,
 // a block per image plane:
@@ -20,10 +20,11 @@
 //   is what most of the instructions are for (two 64-bit mixes, a logarithm, a
 //   root and a cosine per pixel); a last pass applies contrast, noise, clamp
 //   and erasing and stores.
-// Larger ones go through global memory between three kernels (affine, plane
-// means, pixels).  Measured at 2048 x 28 x 28 with everything on: the three
-// kernels and the table's upload took 58 us, and the host pass with all draws
-// about 45 us per batch.
+// Larger ones go through global memory between four kernels (parameters, affine,
+// plane means, pixels).  Measured at 2048 x 28 x 28 with everything on: the host pass
+// takes 18 us of the call's 27 and the kernel 25 us beside the next batch's host pass;
+// with all draws on the host that pass took 45 us, the three kernels and the upload of
+// its table 58.
 //
 // Arithmetic that the reference rounds step by step is written with the
 // round-to-nearest intrinsics, which the compiler never contracts into fused

@@ -39,7 +39,6 @@ struct AugmentationDraws {
     unsigned long long state;   // stream state before the sample's first draw
     float cosine, sine;         // of the rotation, by the host's libm
     unsigned erase;             // the erasing decision
-    unsigned pad;
 };
 
 bool augmentation_enabled(const AugmentationSettings &settings);

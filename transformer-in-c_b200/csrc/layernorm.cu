@@ -7,8 +7,8 @@
 // recomputes the statistics from x instead of reading saved ones, and folds
 // the gamma / beta gradients (column sums over all rows) into the same pass:
 // each lane keeps running sums for the columns it owns, warps of a block
-// combine through shared memory, and one atomic per column and block lands
-// the result.
+// combine through shared memory, and one reduction per four columns and block
+// lands the result.
 #include "kernels.h"
 #include "device_util.cuh"
 

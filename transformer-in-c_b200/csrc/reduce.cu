@@ -1,5 +1,6 @@
 // Column sums of a row-major matrix: out[c] += sum_r in[r*ld + c].
-// Used for bias gradients and for the positional / CLS gradients.
+// Used for bias gradients and for the positional / CLS gradients; matrices of many
+// columns take column_strips_kernel below.
 //
 // A block owns a strip of columns (32 threads wide, each thread 1 or 4
 // adjacent columns) and a slice of the rows; its 32 row lanes walk the slice
