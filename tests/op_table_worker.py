@@ -168,6 +168,12 @@ def slope_product_errors(case):
     tensors["y"].grad.array()[:] = values["y"].ravel()
     fused = host.backend.fusion_counters()["epilogues"]
     op("gemm_backward", pointer["activated"], pointer["w"], pointer["y"])
+    if "read_under" in case:   # the product is still held back
+        host.backend.set_gemm_precision(case["read_under"])
+        host.options = None
+        want = values["y"].astype(np.float64) @ values["w"].astype(np.float64).T
+        got = tensors["activated"].grad.array().reshape(want.shape)
+        return {"activated": float(np.abs(got - want).max() / np.abs(want).max())}
     op("gelu_backward", pointer["hidden"], pointer["activated"])
     op("bias_add_backward", pointer["hidden"], pointer["bias"])
     host.synchronize()
@@ -196,6 +202,9 @@ def skipped_gradients(case):
     start = counters()
     state.train()
     end = counters()
+    if "read_under" in case:   # another policy by the time they are read
+        state.host.backend.set_gemm_precision(case["read_under"])
+        state.host.options = None
     found["defined"] = (end["lazy_defined"] - start["lazy_defined"]) / case["layers"]
     for layer in range(case["layers"]):
         activated, branch = (

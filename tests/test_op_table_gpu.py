@@ -130,6 +130,18 @@ def test_skipped_gradients_are_those_of_the_weights_before_the_step():
     assert len(found) == len(cases)
 
 
+def test_gradients_computed_later_keep_the_precision_they_were_asked_in():
+    """FP32 products that wait (skipped by the GELU's backward pass, or held back for it)
+    while the host switches to TF32."""
+    tf32 = 2
+    shape = model(1, 28, 4, 64, 4, 1, 11)
+    skipped, held = run([
+        dict(train(4, shape, precision="fp32"), skipped_gradients=True, read_under=tf32),
+        dict(kind="slope_product", m=300, k=256, n=64, read_under=tf32)])
+    assert skipped["before"] <= 2e-5, skipped
+    assert held["activated"] <= 2e-5, held
+
+
 SETTINGS = dict(max_shift_pixels=2.0, max_rotation_degrees=10.0, max_scale_delta=0.1,
                 max_brightness_delta=0.05, max_contrast_delta=0.1,
                 noise_standard_deviation=0.01, erasing_probability=0.5,

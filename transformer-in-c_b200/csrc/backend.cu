@@ -167,11 +167,13 @@ struct PendingInputGradient {
     bool active = false;
     const void *dx_host = nullptr, *w_host = nullptr, *dy_host = nullptr;
     int m = 0, k = 0, n = 0;
+    int precision = 0;   // as below
 };
 
 // Arguments of a gradient that was skipped that way, should somebody read it.
 struct InputGradientShape {
     int m, k, n;
+    int precision;   // FP32, or TF32 where the layout allows
 };
 
 // A batch's augmentation plan in page-locked memory, and when it has been read.
@@ -509,6 +511,16 @@ float *accumulate_view(CudaBackend *backend, const void *pointer, bool *add) {
     return device;
 }
 
+// dX (+)= dY W^T under the policy that held when the host asked for it (the product may
+// run much later, see gelu_backward_through_product).
+void input_gradient(const float *w, const float *dy, float *dx, int m, int k, int n,
+                    int precision, bool add, cudaStream_t stream) {
+    if (gemm_backward_input(w, dy, dx, m, k, n, precision, add, stream) != 0 &&
+        precision == VITB200_PRECISION_TF32) {
+        gemm_backward_input(w, dy, dx, m, k, n, VITB200_PRECISION_FP32, add, stream);
+    }
+}
+
 // dX = dY W^T on its own: the op after the product's backward pass was not
 // the GELU backward pass the product was held back for.
 void flush_input_gradient(CudaBackend *backend) {
@@ -522,8 +534,8 @@ void flush_input_gradient(CudaBackend *backend) {
                   4.0 * (double(held.m) * held.n + double(held.k) * held.n +
                          (add ? 2.0 : 1.0) * double(held.m) * held.k),
                   2.0 * double(held.m) * held.k * held.n);
-    gemm_backward_input(w, dy, dx, held.m, held.k, held.n,
-                        VITB200_PRECISION_AUTO, add, backend->stream);
+    input_gradient(w, dy, dx, held.m, held.k, held.n, held.precision, add,
+                   backend->stream);
 }
 
 
@@ -887,6 +899,7 @@ int op_gemm_backward(void *context, vitb200_tensor *left, vitb200_tensor *right,
         held.m = m;
         held.k = k;
         held.n = n;
+        held.precision = gemm_chosen_precision(double(m) * k * n);
         dp_gradient_produced(backend->dp, right->grad, dw, numel(right));
         return 0;
     }
@@ -1251,8 +1264,8 @@ void materialise_input_gradient(const void *arguments, float *output,
                                 float *const *sources, cudaStream_t stream) {
     InputGradientShape shape;
     memcpy(&shape, arguments, sizeof(shape));
-    gemm_backward_input(sources[1], sources[0], output, shape.m, shape.k,
-                        shape.n, VITB200_PRECISION_AUTO, false, stream);
+    input_gradient(sources[1], sources[0], output, shape.m, shape.k, shape.n,
+                   shape.precision, false, stream);
 }
 
 // gelu_backward right after the gemm_backward that would have produced its
@@ -1279,7 +1292,7 @@ bool gelu_backward_through_product(CudaBackend *backend,
     const float *w = view(backend, held.w_host, Access::Read);
     const float *dy = view(backend, held.dy_host, Access::Read);
     const float *h = view(backend, input->data, Access::Read);
-    const InputGradientShape shape = {held.m, held.k, held.n};
+    const InputGradientShape shape = {held.m, held.k, held.n, held.precision};
     if (!coherent_define_lazy(held.dx_host, sources, 2,
                               materialise_input_gradient, &shape, sizeof(shape),
                               backend->stream)) {
@@ -1298,7 +1311,7 @@ bool gelu_backward_through_product(CudaBackend *backend,
                              2.0 * double(held.m) * held.k),
                       2.0 * double(held.m) * held.k * held.n);
         if (gemm_backward_input_gelu(w, dy, h, dh, sums, held.m, held.k, held.n,
-                                     VITB200_PRECISION_AUTO, backend->stream,
+                                     held.precision, backend->stream,
                                      &partial_rows) != 0) {
             fprintf(stderr, "vitb200: fused product + GELU backward failed to launch\n");
             abort();

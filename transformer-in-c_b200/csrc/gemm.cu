@@ -93,6 +93,12 @@ int gemm_default_precision() {
     return default_precision();
 }
 
+int gemm_chosen_precision(double multiply_adds) {
+    return prefer_tensor_cores(VITB200_PRECISION_AUTO, multiply_adds)
+        ? VITB200_PRECISION_TF32
+        : VITB200_PRECISION_FP32;
+}
+
 bool prefer_tensor_cores(int precision, double multiply_adds) {
     if (precision == VITB200_PRECISION_AUTO) {
         precision = default_precision();

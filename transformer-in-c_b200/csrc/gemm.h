@@ -65,6 +65,10 @@ bool prefer_tensor_cores(int precision, double multiply_adds);
 // when no override is active).
 int gemm_default_precision();
 
+// What a product of `multiply_adds` gets under the policy of this moment: FP32, or
+// TF32 (where the layout allows).  For products that run later than they are asked for.
+int gemm_chosen_precision(double multiply_adds);
+
 // Overrides what VITB200_PRECISION_AUTO means (and the VITB200_GEMM
 // environment variable); -1 restores the default policy.
 void gemm_set_default_precision(int precision);
