@@ -188,6 +188,41 @@ def slope_product_errors(case):
     return found
 
 
+def gradient_pair_errors(case):
+    """Both gradients of a product, twice (the weights' add up, the input's starts from
+    zero again): largest errors against the largest entry, and the kernels of the second
+    pass."""
+    rng = np.random.default_rng(case["m"])
+    host, m, k, n = cases._the_host(), case["m"], case["k"], case["n"]
+    host.configure({"precision": case["precision"], "deferred": False})
+    tensors = {name: cases._Tensor(*shape) for name, shape in (
+        ("x", (m, k)), ("w", (k, n)), ("y", (m, n)))}
+    values = {name: rng.standard_normal((t.rows, t.cols)).astype(np.float32)
+              for name, t in tensors.items()}
+    pointer = {name: t.pointer for name, t in tensors.items()}
+
+    def op(slot, *arguments):
+        assert host.ops[slot](host.table_context, *arguments) == 0, slot
+
+    for name in ("x", "w"):
+        tensors[name].array()[:] = values[name]
+    kept = cases._pointers([pointer["x"], pointer["w"]])
+    op("zero_gradients", ctypes.addressof(kept), 2)
+    tensors["y"].grad.array()[:] = values["y"].ravel()
+    for _ in range(2):
+        op("zero_gradient", pointer["x"])
+        host.synchronize()
+        launches = host.backend.kernel_launches()
+        op("gemm_backward", pointer["x"], pointer["w"], pointer["y"])
+        host.synchronize()
+    found = {"kernels": host.backend.kernel_launches() - launches}
+    x, w, dy = (values[name].astype(np.float64) for name in ("x", "w", "y"))
+    for name, want in (("x", dy @ w.T), ("w", 2.0 * (x.T @ dy))):
+        got = tensors[name].grad.array().reshape(want.shape)
+        found[name] = float(np.abs(got - want).max() / np.abs(want).max())
+    return found
+
+
 def skipped_gradients(case):
     """The gradients of the GELU outputs, which no kernel stores, read after the
     optimiser has moved the weights they are defined by: largest error against
@@ -223,6 +258,8 @@ def skipped_gradients(case):
 def errors(case):
     if case["kind"] == "slope_product":
         return slope_product_errors(case)
+    if case["kind"] == "gradient_pair":
+        return gradient_pair_errors(case)
     if case["kind"] == "gelu_parameter":
         return gelu_parameter_errors()
     if case["kind"] == "augment":

@@ -115,6 +115,27 @@ def test_slope_products_on_the_fma_tiles():
         assert all(error <= 2e-5 for error in errors.values()), (case, errors)
 
 
+def test_gradients_of_small_products_share_a_launch():
+    """One row, ragged tiles, slices in a cluster beside more or fewer weight slices;
+    tensor-core tiles of 32 and of 64 columns with ragged edges, and products that are
+    too large to run side by side.  Bounds as for the products."""
+    def cases(precision, *sizes):
+        return [dict(kind="gradient_pair", precision=precision, m=m, k=k, n=n)
+                for m, k, n in sizes]
+    small = cases("fp32", (1, 5, 3), (50, 512, 128), (50, 33, 11), (8, 128, 11),
+                  (257, 40, 129), (1000, 32, 96))
+    narrow = cases("auto", (1600, 128, 512), (1600, 512, 128), (1601, 100, 388),
+                   (4329, 96, 384), (4329, 384, 96), (25, 1024, 1024))
+    large = cases("auto", (20000, 128, 512), (9000, 512, 64)) + \
+        cases("fp32", (9000, 16, 128))
+    found = run(small + narrow + large)
+    assert len(found) == len(small + narrow + large)
+    for case, errors in zip(small + narrow + large, found):
+        assert errors.pop("kernels") == (2 if case in large else 1), (case, errors)
+        bound = 2e-5 if case["precision"] == "fp32" else 2e-3
+        assert all(error <= bound for error in errors.values()), (case, errors)
+
+
 def test_skipped_gradients_are_those_of_the_weights_before_the_step():
     """Bounds as for the products (FP32 2e-5, TF32 2e-3 of the largest entry); a step
     moves the weights by about a hundredth of themselves.  Definitions of a block and

@@ -219,4 +219,32 @@ int gemm_backward_input_gelu(const float *w, const float *dy,
     return launch_gemm_fma(f, stream, partial_rows);
 }
 
+bool gemm_backward_pairs(int m, int k, int n, int precision) {
+    return prefer_tensor_cores(precision, double(m) * k * n) ? gemm_tc_pairs(m, k, n)
+                                                            : gemm_fma_pairs(m, k, n);
+}
+
+bool gemm_backward_pair(const float *x, const float *w, const float *dy, float *dx,
+                        float *dw, const float *gelu_input, float *column_partials,
+                        int m, int k, int n, int precision, cudaStream_t stream,
+                        int *partial_rows) {
+    TcGemm gx = {dy, w, dx, nullptr, m, k, n, n, n, k, false, false, false};
+    gx.gelu_input = gelu_input;
+    gx.ld_gelu_input = gelu_input ? k : 0;
+    gx.column_partials = column_partials;
+    TcGemm gw = {x, dy, dw, nullptr, k, n, m, k, n, n, true, true, true};
+    const int input = use_tensor_cores(gx, precision);
+    if (input < 0 || input != use_tensor_cores(gw, precision)) {
+        return false;
+    }
+    if (input == 1) {
+        return launch_gemm_tc_pair(gx, gw, stream, partial_rows) == 0;
+    }
+    FmaGemm fx = fma_form(gx);
+    fx.gelu_input = gelu_input;
+    fx.column_partials = column_partials;
+    fx.partial_row_limit = kGemmPartialRows;
+    return launch_gemm_fma_pair(fx, fma_form(gw), stream, partial_rows) == 0;
+}
+
 }  // namespace vitb200

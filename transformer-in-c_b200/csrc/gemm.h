@@ -51,6 +51,16 @@ int gemm_backward_input_gelu(const float *w, const float *dy,
                              float *column_partials, int m, int k, int n,
                              int precision, cudaStream_t stream,
                              int *partial_rows);
+// Both halves in one launch, for products so small that a launch costs more than its
+// work: dX is stored, not added to, and multiplied by gelu'(gelu_input) where that is
+// given (with column_partials as above), dW is added to.  gemm_backward_pairs says
+// whether the sizes are in that range; false, with nothing launched, where a layout
+// is not served.
+bool gemm_backward_pairs(int m, int k, int n, int precision);
+bool gemm_backward_pair(const float *x, const float *w, const float *dy, float *dx,
+                        float *dw, const float *gelu_input, float *column_partials,
+                        int m, int k, int n, int precision, cudaStream_t stream,
+                        int *partial_rows);
 // Whether that product runs on the tensor cores.
 bool gemm_backward_input_gelu_on_tensor_cores(const float *w, const float *dy,
                                               const float *gelu_input,

@@ -260,10 +260,10 @@ struct Operand {
 // A_K / B_K: the operand's rows have K contiguous (otherwise M / N).
 // CLUSTER: blockIdx.z runs over the K slices of one tile, which are the CTAs
 // of a cluster and add up through distributed shared memory.
-template <int TM, int TN, int RM, int RN, int KB, int CTAS, bool A_K, bool B_K,
-          bool CLUSTER>
-__global__ void __launch_bounds__(TM / RM * (TN / RN), CTAS)
-fma_kernel(const FmaParams p) {
+// place: the CTA's tile (x, y) and slice (z) of `slices`.
+template <int TM, int TN, int RM, int RN, int KB, bool A_K, bool B_K, bool CLUSTER>
+__device__ __forceinline__ void fma_tile(const FmaParams &p, const uint3 place,
+                                         const int slices) {
     constexpr int kThreads = TM / RM * (TN / RN);
     constexpr int kLanesX = TN / RN, kLanesY = TM / RM;
     static_assert(kLanesX % 4 == 0 && kLanesY % 8 == 0 && RM % 4 == 0, "warp = 8 x 4 threads");
@@ -276,9 +276,9 @@ fma_kernel(const FmaParams p) {
     const int lane = tid & 31, warp = tid >> 5;
     const int ty = (warp / (kLanesX / 4)) * 8 + (lane & 7);
     const int tx = (warp % (kLanesX / 4)) * 4 + (lane >> 3);
-    const int m0 = blockIdx.x * TM;
-    const int n0 = blockIdx.y * TN;
-    const int k_begin = blockIdx.z * p.k_per_split;
+    const int m0 = int(place.x) * TM;
+    const int n0 = int(place.y) * TN;
+    const int k_begin = int(place.z) * p.k_per_split;
     const int k_end = min(p.k, k_begin + p.k_per_split);
     const int blocks = k_end > k_begin ? (k_end - k_begin + KB - 1) / KB : 0;
 
@@ -370,8 +370,8 @@ fma_kernel(const FmaParams p) {
             column_sums[c] = 0.0f;
         }
     }
-    int partial_row = blockIdx.x;
-    if (CLUSTER && gridDim.z > 1) {
+    int partial_row = place.x;
+    if (CLUSTER && slices > 1) {
         // Every CTA of the cluster leaves its partial tile in its own shared
         // memory and finishes an equal share of the rows.
         constexpr int kPitch = TN + 4;
@@ -386,9 +386,9 @@ fma_kernel(const FmaParams p) {
         }
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-        const int slices = gridDim.z, rank = blockIdx.z;
+        const int rank = place.z;
         const int rows = TM / slices;
-        partial_row = blockIdx.x * slices + rank;
+        partial_row = place.x * slices + rank;
         for (int e = tid; e < rows * TN; e += kThreads) {
             const int r = rank * rows + e / TN, c = e % TN;
             const uint32_t mine = shared_address(shared + r * kPitch + c);
@@ -460,6 +460,42 @@ fma_kernel(const FmaParams p) {
             }
         }
     }
+}
+
+template <int TM, int TN, int RM, int RN, int KB, int CTAS, bool A_K, bool B_K,
+          bool CLUSTER>
+__global__ void __launch_bounds__(TM / RM * (TN / RN), CTAS)
+fma_kernel(const FmaParams p) {
+    fma_tile<TM, TN, RM, RN, KB, A_K, B_K, CLUSTER>(p, blockIdx, int(gridDim.z));
+}
+
+// The smallest tile, with which latency-sized products run.
+constexpr int kSmallRows = 32, kSmallCols = 32, kSmallRm = 4, kSmallRn = 2, kSmallKb = 32;
+
+// The two gradients of a small linear layer side by side, each as a launch of its own
+// would compute it.  Tiles of the input gradient first (p, x_tiles x y_tiles of them,
+// their slices along z a cluster), then the weight gradient's (q) tiles and slices,
+// numbered through.
+__global__ void __launch_bounds__(kSmallRows / kSmallRm * (kSmallCols / kSmallRn), 4)
+fma_pair_kernel(const FmaParams p, const FmaParams q, const unsigned x_tiles,
+                const unsigned y_tiles, const unsigned x_weight, const unsigned y_weight,
+                const unsigned weight_slices) {
+    const unsigned tiles = x_tiles * y_tiles;
+    if (blockIdx.x < tiles) {
+        fma_tile<kSmallRows, kSmallCols, kSmallRm, kSmallRn, kSmallKb, true, true, true>(
+            p, make_uint3(blockIdx.x % x_tiles, blockIdx.x / x_tiles, blockIdx.z),
+            int(gridDim.z));
+        return;
+    }
+    const unsigned index = (blockIdx.x - tiles) * gridDim.z + blockIdx.z;
+    const unsigned weight_tiles = x_weight * y_weight;
+    if (index >= weight_tiles * weight_slices) {
+        grid_dependency_wait();
+        return;
+    }
+    const unsigned tile = index % weight_tiles;
+    fma_tile<kSmallRows, kSmallCols, kSmallRm, kSmallRn, kSmallKb, false, false, false>(
+        q, make_uint3(tile % x_weight, tile / x_weight, index / weight_tiles), 1);
 }
 
 enum class Form { Forward, InputGradient, WeightGradient };
@@ -612,12 +648,18 @@ bool aligned16(const void *pointer) {
 
 unsigned long long g_fma_products = 0;
 
-int launch_gemm_fma(const FmaGemm &g, cudaStream_t stream, int *partial_rows) {
-    if (launch_gemm_thin(g, stream)) {
-        ++g_fma_products;
-        return 0;
-    }
-    FmaParams p = {};
+namespace {
+
+// A product with its plan, ready to be launched.
+struct FmaLaunch {
+    FmaParams p;
+    Form form;
+    int tile, slices;
+};
+
+bool prepare(const FmaGemm &g, cudaStream_t stream, int *partial_rows, FmaLaunch *out) {
+    FmaParams &p = out->p;
+    p = FmaParams{};
     p.a = g.a;
     p.b = g.b;
     p.c = g.c;
@@ -639,7 +681,7 @@ int launch_gemm_fma(const FmaGemm &g, cudaStream_t stream, int *partial_rows) {
     const Form form = g.a_k ? (g.b_k ? Form::InputGradient : Form::Forward)
                             : Form::WeightGradient;
     if (form == Form::WeightGradient && (!g.accumulate || g.b_k)) {
-        return -1;   // no caller has this form
+        return false;   // no caller has this form
     }
     // K slices may only add into C.
     const bool adds = g.accumulate && form != Form::Forward;
@@ -661,14 +703,34 @@ int launch_gemm_fma(const FmaGemm &g, cudaStream_t stream, int *partial_rows) {
         if (p.partials_shared &&
             cudaMemsetAsync(p.partials, 0, size_t(p.partial_rows) * g.n * sizeof(float),
                             stream) != cudaSuccess) {
-            return -1;
+            return false;
         }
         if (partial_rows) {
             *partial_rows = p.partial_rows;
         }
     }
+    out->form = form;
+    out->tile = plan.tile;
+    out->slices = slices;
+    return true;
+}
+
+}  // namespace
+
+int launch_gemm_fma(const FmaGemm &g, cudaStream_t stream, int *partial_rows) {
+    if (launch_gemm_thin(g, stream)) {
+        ++g_fma_products;
+        return 0;
+    }
+    FmaLaunch launch;
+    if (!prepare(g, stream, partial_rows, &launch)) {
+        return -1;
+    }
+    const FmaParams &p = launch.p;
+    const Form form = launch.form;
+    const int slices = launch.slices;
     cudaError_t status;
-    switch (plan.tile) {
+    switch (launch.tile) {
     case 0:
         status = launch_tile<128, 128, 8, 8, 16, 2>(p, form, slices, stream);
         break;
@@ -682,12 +744,57 @@ int launch_gemm_fma(const FmaGemm &g, cudaStream_t stream, int *partial_rows) {
         status = launch_tile<64, 32, 4, 4, 32, 4>(p, form, slices, stream);
         break;
     default:
-        status = launch_tile<32, 32, 4, 2, 32, 4, true>(p, form, slices, stream);
+        status = launch_tile<kSmallRows, kSmallCols, kSmallRm, kSmallRn, kSmallKb, 4, true>(
+            p, form, slices, stream);
     }
     if (status != cudaSuccess) {
         return -1;
     }
     ++g_fma_products;
+    ++g_kernel_launches;
+    return 0;
+}
+
+bool gemm_fma_pairs(int m, int k, int n) {
+    if (m >= 8192) {
+        return false;   // from here on thin products have kernels of their own
+    }
+    const FmaPlan input = plan_product(m, k, n, false, true, LLONG_MAX);
+    const FmaPlan weight = plan_addition(k, n, m, false);
+    return input.tile == kSmallestTile && weight.tile == kSmallestTile;
+}
+
+int launch_gemm_fma_pair(const FmaGemm &input, const FmaGemm &weight, cudaStream_t stream,
+                         int *partial_rows) {
+    FmaLaunch first, second;
+    if (input.accumulate || !gemm_fma_pairs(input.m, input.n, input.k) ||
+        !prepare(input, stream, partial_rows, &first) ||
+        !prepare(weight, stream, nullptr, &second) ||
+        first.form != Form::InputGradient || second.form != Form::WeightGradient ||
+        first.tile != kSmallestTile || second.tile != kSmallestTile) {
+        return -1;
+    }
+    constexpr int kPairThreads = kSmallRows / kSmallRm * (kSmallCols / kSmallRn);
+    constexpr size_t kBytes =
+        size_t(kStages) * sizeof(float) * 2 *
+        Operand<kSmallRows, kSmallKb, kPairThreads, true>::kFloats;
+    static_assert(kSmallRows == kSmallCols &&
+                      kBytes >= size_t(kSmallRows) * (kSmallCols + 4) * sizeof(float) &&
+                      kBytes <= 40 * 1024,
+                  "one ring for both forms and for the partial tiles");
+    const unsigned x = (first.p.m + kSmallRows - 1) / kSmallRows;
+    const unsigned y = (first.p.n + kSmallCols - 1) / kSmallCols;
+    const unsigned xw = (second.p.m + kSmallRows - 1) / kSmallRows;
+    const unsigned yw = (second.p.n + kSmallCols - 1) / kSmallCols;
+    const unsigned depth = unsigned(first.slices);
+    const unsigned weight_blocks = (xw * yw * unsigned(second.slices) + depth - 1) / depth;
+    const dim3 grid(x * y + weight_blocks, 1, depth);
+    if (launch_chained_cluster(fma_pair_kernel, grid, kPairThreads, kBytes, depth, true,
+                               stream, first.p, second.p, x, y, xw, yw,
+                               unsigned(second.slices)) != cudaSuccess) {
+        return -1;
+    }
+    g_fma_products += 2;
     ++g_kernel_launches;
     return 0;
 }

@@ -91,7 +91,7 @@ constexpr int kSecondResidual = 2;   // D = A*B + bias, D2 = D + residual
 constexpr int kGeluSlope = 3;
 
 // Persistent kernel: each CTA walks work items (output tile x reduction
-// slice) item = blockIdx.x, blockIdx.x + gridDim.x, ...; the three roles run
+// slice) item = cta, cta + ctas, ...; the three roles run
 // the same sequence and meet only through mbarriers, so the loads and MMAs of
 // item i+1 overlap the epilogue of item i (two accumulator buffers in TMEM).
 //
@@ -111,12 +111,11 @@ constexpr int kGeluSlope = 3;
 // start on half 0 while half 1 is still being drained.
 // SECOND is the epilogue variant (0 or a kSecond... / kGeluSlope constant): a
 // compile-time choice, so that no variant pays for another's registers.
+// `cta` of `ctas`: this CTA's place among those that walk the product's items.
 template <int TILE_M, int TILE_N, int SECOND>
-__global__ void __launch_bounds__(TILE_M == 2 * kTileM ? kThreadsTall : kThreads)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
-               const __grid_constant__ CUtensorMap map_b,
-               const __grid_constant__ CUtensorMap map_d,
-               const __grid_constant__ CUtensorMap map_d2, const TcParams p) {
+__device__ __forceinline__ void
+walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorMap &map_d,
+             const CUtensorMap &map_d2, const TcParams &p, const int cta, const int ctas) {
     // All shared memory is dynamic, so that it starts at the beginning of the
     // CTA's window and the swizzled tiles get their 1024-byte alignment without
     // padding (two CTAs with three stages each fill the SM to the last KiB):
@@ -185,7 +184,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
     if (SECOND == kGeluSlope && p.column_partials) {
         // This CTA's own row of column sums, which its epilogue warps add into.
         for (int c = threadIdx.x; c < p.n; c += blockDim.x) {
-            p.column_partials[size_t(blockIdx.x) * p.n + c] = 0.0f;
+            p.column_partials[size_t(cta) * p.n + c] = 0.0f;
         }
         __threadfence();
         __syncthreads();
@@ -197,7 +196,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
     if (warp == 0) {
         if (lane == 0) {
             int fill = 0;   // k-blocks loaded so far, across items
-            for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+            for (int item = cta; item < items && ok; item += ctas) {
                 const int tile = item % tiles;
                 const int m0 = (tile / p.n_tiles) * TILE_M;
                 const int n0 = (tile % p.n_tiles) * TILE_N;
@@ -260,8 +259,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
                 p.b_mn_major ? kLayoutSwizzle128Base32 : kLayoutSwizzle128;
             int drain = 0;   // k-blocks consumed so far, across items
             int local = 0;   // items processed by this CTA
-            for (int item = blockIdx.x; item < items && ok;
-                 item += gridDim.x, ++local) {
+            for (int item = cta; item < items && ok;
+                 item += ctas, ++local) {
                 const int tile_splits = item / tiles;
                 const int n_live = min(TILE_N, p.n - ((item % tiles) % p.n_tiles) * TILE_N);
                 const uint32_t idesc =
@@ -352,11 +351,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
             }
             ++issued;
         };
-        if (int(blockIdx.x) < items) {
-            request(blockIdx.x, 0);
+        if (cta < items) {
+            request(cta, 0);
         }
         int local = 0;
-        for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++local) {
+        for (int item = cta; item < items && ok; item += ctas, ++local) {
             const int tile = item % tiles;
             const int m0 = (tile / p.n_tiles) * kTileM + quarter * 32;
             const int n0 = (tile % p.n_tiles) * TILE_N;
@@ -389,8 +388,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
                 // The block after this one, possibly the next tile's first.
                 if (chunk + 1 < TILE_N / 32) {
                     request(item, chunk + 1);
-                } else if (item + int(gridDim.x) < items) {
-                    request(item + gridDim.x, 0);
+                } else if (item + ctas < items) {
+                    request(item + ctas, 0);
                 }
                 if (!chunk_live) {
                     continue;   // uniform across the warp
@@ -428,7 +427,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
                                      (lane & 3)];
                     }
                     if (col0 + lane < p.n) {
-                        atomicAdd(p.column_partials + size_t(blockIdx.x) * p.n +
+                        atomicAdd(p.column_partials + size_t(cta) * p.n +
                                       col0 + lane,
                                   sum);
                     }
@@ -464,7 +463,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
             : staging + quarter * (p.staging_bytes / 4);
         int local = 0;
         int stored = 0;   // blocks handed to TMA so far (selects the buffer)
-        for (int item = blockIdx.x; item < items; item += gridDim.x, ++local) {
+        for (int item = cta; item < items; item += ctas, ++local) {
             const int tile = item % tiles;
             const int m0 = (tile / p.n_tiles) * TILE_M + half * kTileM + quarter * 32;
             const int n0 = (tile % p.n_tiles) * TILE_N;
@@ -663,6 +662,38 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
     }
 }
 
+template <int TILE_M, int TILE_N, int SECOND>
+__global__ void __launch_bounds__(TILE_M == 2 * kTileM ? kThreadsTall : kThreads)
+gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
+               const __grid_constant__ CUtensorMap map_b,
+               const __grid_constant__ CUtensorMap map_d,
+               const __grid_constant__ CUtensorMap map_d2, const TcParams p) {
+    walk_product<TILE_M, TILE_N, SECOND>(map_a, map_b, map_d, map_d2, p, blockIdx.x,
+                                         gridDim.x);
+}
+
+// Two independent products side by side: the gradients of one linear layer when
+// both are so small that a launch of their own costs more than their work.  The
+// first `ctas` CTAs walk the input gradient (with the GELU slope or without), the
+// others the weight gradient.
+struct TcPairMaps {
+    CUtensorMap a, b, d, d2;
+};
+
+template <int TILE_N, int SECOND>
+__global__ void __launch_bounds__(kThreads)
+gemm_tc_pair_kernel(const __grid_constant__ TcPairMaps input,
+                    const __grid_constant__ TcPairMaps weight, const TcParams p,
+                    const TcParams q, const int ctas) {
+    if (int(blockIdx.x) < ctas) {
+        walk_product<kTileM, TILE_N, SECOND>(input.a, input.b, input.d, input.d2, p,
+                                             blockIdx.x, ctas);
+    } else {
+        walk_product<kTileM, TILE_N, 0>(weight.a, weight.b, weight.d, weight.d, q,
+                                        blockIdx.x - ctas, gridDim.x - ctas);
+    }
+}
+
 // ---- host side -------------------------------------------------------------
 
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t,
@@ -842,12 +873,52 @@ bool gemm_tc_supported(const TcGemm &g) {
            encode_tiled();
 }
 
-int launch_gemm_tc(const TcGemm &g, cudaStream_t stream, int *partial_rows) {
-    if (!gemm_tc_supported(g)) {
-        return -1;
+namespace {
+
+// Long reductions onto few output tiles (weight gradients) are cut into slices.
+// With a persistent grid the slices should fill the CTA slots evenly: picks the slice
+// count that minimises the k-blocks the busiest CTA walks (*walked), charging each item
+// about eight k-blocks for its epilogue and reduce-add.
+int choose_slices(long long tiles, int k_blocks, long long slots, long long *walked) {
+    long long best_cost = -1;
+    int slices = 1;
+    for (int candidate = 1; candidate <= 512; ++candidate) {
+        const int per_slice = (k_blocks + candidate - 1) / candidate;
+        if (candidate > 1 && per_slice < 4) {
+            break;
+        }
+        const long long rounds = (tiles * candidate + slots - 1) / slots;
+        if (best_cost >= 0 && rounds * (4 + 8) >= best_cost) {
+            break;   // more slices take no fewer rounds
+        }
+        const long long cost = rounds * (per_slice + 8);
+        if (best_cost < 0 || cost < best_cost) {
+            best_cost = cost;
+            slices = candidate;
+        }
     }
-    if (!raise_limits()) {
-        return -1;
+    if (walked) {
+        *walked = best_cost;
+    }
+    return slices;
+}
+
+// A product ready to be launched.
+struct TcLaunch {
+    const TcTile *tile;
+    int second;
+    TcPairMaps maps;
+    TcParams p;
+    unsigned grid;
+    int smem_bytes;
+};
+
+// Fills in `out`; false when the product cannot be served.  forced_narrow: one of the
+// narrow tiles instead of the choice below, with at most `most_ctas` CTAs (the other
+// product of a pair has the rest of the SMs).
+bool prepare(const TcGemm &g, int forced_narrow, long long most_ctas, TcLaunch *out) {
+    if (!gemm_tc_supported(g) || !raise_limits()) {
+        return false;
     }
     // Wide tiles where the product is compute-bound: deep reductions, one
     // output (or the GELU pair), a multiple of 128 columns.
@@ -903,8 +974,8 @@ int launch_gemm_tc(const TcGemm &g, cudaStream_t stream, int *partial_rows) {
     // (13 tiles before, 52 now), [1600,128]x[128,512] 7.6 -> 5.6 us, with GELU
     // 10.4 -> 7.8; a step of batch 32 762 -> 668 us, of 117 colour images
     // 559 -> 530 us.  With one tile per SM as the limit these were 673 and 542.
-    int narrow = -1;
-    if (!g.residual && !forced_tile && !forced_tile_m) {
+    int narrow = forced_narrow;
+    if (narrow < 0 && !g.residual && !forced_tile && !forced_tile_m) {
         const long long row_tiles = (g.m + kTileM - 1) / kTileM;
         // (The slices of a split reduction, four blocks each at least.)
         const long long slices =
@@ -923,11 +994,11 @@ int launch_gemm_tc(const TcGemm &g, cudaStream_t stream, int *partial_rows) {
     const int tile_m = tile.m, tile_n = tile.n;
     const int second = g.d2 ? (g.residual ? kSecondResidual : kSecondGelu)
                             : (g.gelu_input ? kGeluSlope : 0);
-    const TcKernel kernel = tile.kernel(second);
-    if (!kernel) {
-        return -1;
+    if (!tile.kernel(second)) {
+        return false;
     }
-    CUtensorMap map_a, map_b, map_d;
+    CUtensorMap &map_a = out->maps.a, &map_b = out->maps.b, &map_d = out->maps.d,
+                &map_d2 = out->maps.d2;
     // K-major operand: rows = output index, inner = reduction index.
     // MN-major operand: rows = reduction index, inner = output index.
     const CUtensorMapSwizzle chunks16 = CU_TENSOR_MAP_SWIZZLE_128B;
@@ -940,18 +1011,18 @@ int launch_gemm_tc(const TcGemm &g, cudaStream_t stream, int *partial_rows) {
         : tensor_map(g.b, g.k, g.n, g.ldb, 32, tile_n, chunks16, true, &map_b);
     const bool ok_d =
         tensor_map(g.d, g.n, g.m, g.ldd, 32, 32, chunks16, false, &map_d);
-    CUtensorMap map_d2 = map_d;
+    map_d2 = map_d;
     const bool ok_d2 = !g.d2 ||
         tensor_map(g.d2, g.n, g.m, g.ldd2, 32, 32, chunks16, false, &map_d2);
     if (!ok_a || !ok_b || !ok_d || !ok_d2) {
-        return -1;
+        return false;
     }
     if (g.gelu_input &&
         !tensor_map(g.gelu_input, g.n, g.m, g.ld_gelu_input, 32, 32, chunks16,
                     false, &map_d2)) {
-        return -1;
+        return false;
     }
-    TcParams p;
+    TcParams &p = out->p;
     p.m = g.m;
     p.n = g.n;
     p.k_blocks = (g.k + kBlockK - 1) / kBlockK;
@@ -999,7 +1070,8 @@ int launch_gemm_tc(const TcGemm &g, cudaStream_t stream, int *partial_rows) {
         staging_bytes = 2 * kOperandBytes;
     }
     const bool narrowed = tile_n < kTileN;
-    const bool spread = narrowed && (long long)tiles <= (long long)device_sm_count();
+    const bool spread = narrowed && forced_narrow < 0 &&
+                        (long long)tiles <= (long long)device_sm_count();
     if (narrowed && forced_stages == 0) {
         // The ring as deep as the reduction, where a CTA has the SM to itself.
         const int depth = spread && !g.accumulate ? kMaxStages : 4;
@@ -1021,28 +1093,11 @@ int launch_gemm_tc(const TcGemm &g, cudaStream_t stream, int *partial_rows) {
     // One or two persistent CTAs on every multiprocessor (never more than
     // the per-CTA partial rows provide for).
     const long long slots =
-        std::min<long long>((long long)device_sm_count() * ctas_per_sm, kGemmPartialRows);
+        std::min<long long>({(long long)device_sm_count() * ctas_per_sm, kGemmPartialRows,
+                             most_ctas});
     int splits = 1;
     if (g.accumulate) {
-        // Long reductions onto few output tiles (weight gradients) are cut
-        // into slices.  With a persistent grid the slices should fill the CTA
-        // slots evenly: pick the slice count that minimises the k-blocks the
-        // busiest CTA walks, charging each item about eight k-blocks for its
-        // epilogue and reduce-add.
-        long long best_cost = -1;
-        for (int candidate = 1; candidate <= 512; ++candidate) {
-            const int per_slice = (p.k_blocks + candidate - 1) / candidate;
-            if (candidate > 1 && per_slice < 4) {
-                break;
-            }
-            const long long rounds =
-                ((long long)tiles * candidate + slots - 1) / slots;
-            const long long cost = rounds * (per_slice + 8);
-            if (best_cost < 0 || cost < best_cost) {
-                best_cost = cost;
-                splits = candidate;
-            }
-        }
+        splits = choose_slices(tiles, p.k_blocks, slots, nullptr);
     }
     p.k_blocks_per_split = (p.k_blocks + splits - 1) / splits;
     splits = (p.k_blocks + p.k_blocks_per_split - 1) / p.k_blocks_per_split;
@@ -1063,20 +1118,113 @@ int launch_gemm_tc(const TcGemm &g, cudaStream_t stream, int *partial_rows) {
     const long long items = (long long)tiles * splits;
     const int stage_bytes = (tile_m + tile_n) * kBlockK * 4;
     const int smem_bytes = p.stages * stage_bytes + staging_bytes + kBarrierBytes;
-    const unsigned grid = unsigned(items < slots ? items : slots);
-    if (g.column_partials && grid > unsigned(kGemmPartialRows)) {
+    out->grid = unsigned(items < slots ? items : slots);
+    out->smem_bytes = smem_bytes;
+    out->tile = &tile;
+    out->second = second;
+    return true;
+}
+
+}  // namespace
+
+int launch_gemm_tc(const TcGemm &g, cudaStream_t stream, int *partial_rows) {
+    TcLaunch launch;
+    if (!prepare(g, -1, kGemmPartialRows, &launch)) {
         return -1;
     }
     if (g.column_partials && partial_rows) {
-        *partial_rows = int(grid);
+        *partial_rows = int(launch.grid);
     }
-    launch_chained(kernel, grid, tile.threads, smem_bytes, stream, map_a, map_b, map_d,
-                   map_d2, p);
+    const TcPairMaps &maps = launch.maps;
+    launch_chained(launch.tile->kernel(launch.second), launch.grid, launch.tile->threads,
+                   launch.smem_bytes, stream, maps.a, maps.b, maps.d, maps.d2, launch.p);
     ++g_kernel_launches;
     ++g_tc_products;
-    if (tile_n > kTileN) {
+    if (launch.tile->n > kTileN) {
         ++g_tc_wide_products;
     }
+    return 0;
+}
+
+namespace {
+
+// The narrow tile with which the gradients of [m,k] x [k,n] run side by side, or -1:
+// all tiles of the input gradient resident at once with a CTA each, and the weight
+// gradient on the SMs' other slots done no later than the two would be one after the
+// other.  (The gradients of larger products take as long as their work, in one
+// launch or two.)
+int find_pair_tile(int m, int k, int n) {
+    const long long slots = 2LL * device_sm_count();
+    const int depth = (n + kBlockK - 1) / kBlockK;
+    const int weight_depth = (m + kBlockK - 1) / kBlockK;
+    for (int candidate : {kNarrow32, kNarrow64}) {
+        const int width = kTcTiles[candidate].n;
+        const long long first = (m + kTileM - 1LL) / kTileM * ((k + width - 1) / width);
+        const long long second = (k + kTileM - 1LL) / kTileM * ((n + width - 1) / width);
+        if (first + second > slots) {
+            continue;
+        }
+        long long beside = 0, alone = 0;
+        choose_slices(second, weight_depth, slots - first, &beside);
+        choose_slices(second, weight_depth, slots, &alone);
+        if (beside <= depth + 8 + alone) {
+            return candidate;
+        }
+    }
+    return -1;
+}
+
+int pair_tile(int m, int k, int n) {
+    // (Asked before the product is held back and again when it is launched.)
+    static thread_local int last[4] = {0, 0, 0, -1};
+    if (last[0] != m || last[1] != k || last[2] != n) {
+        last[0] = m;
+        last[1] = k;
+        last[2] = n;
+        last[3] = find_pair_tile(m, k, n);
+    }
+    return last[3];
+}
+
+}  // namespace
+
+bool gemm_tc_pairs(int m, int k, int n) {
+    return pair_tile(m, k, n) >= 0;
+}
+
+int launch_gemm_tc_pair(const TcGemm &input, const TcGemm &weight, cudaStream_t stream,
+                        int *partial_rows) {
+    const int tile = pair_tile(input.m, input.n, input.k);
+    if (tile < 0 || input.d2 || weight.d2 || weight.gelu_input || weight.bias) {
+        return -1;
+    }
+    TcLaunch first, second;
+    const long long slots = std::min<long long>(2LL * device_sm_count(), kGemmPartialRows);
+    if (!prepare(input, tile, slots, &first) ||
+        !prepare(weight, tile, slots - first.grid, &second)) {
+        return -1;
+    }
+    const bool slope = first.second == kGeluSlope;
+    const auto kernel = tile == kNarrow32
+        ? (slope ? gemm_tc_pair_kernel<32, kGeluSlope> : gemm_tc_pair_kernel<32, 0>)
+        : (slope ? gemm_tc_pair_kernel<64, kGeluSlope> : gemm_tc_pair_kernel<64, 0>);
+    static SharedMemoryLimit limit;
+    const void *kernels[4] = {
+        reinterpret_cast<const void *>(gemm_tc_pair_kernel<32, 0>),
+        reinterpret_cast<const void *>(gemm_tc_pair_kernel<32, kGeluSlope>),
+        reinterpret_cast<const void *>(gemm_tc_pair_kernel<64, 0>),
+        reinterpret_cast<const void *>(gemm_tc_pair_kernel<64, kGeluSlope>)};
+    if (!limit.raise(kernels, 4, kSmemLimit)) {
+        return -1;
+    }
+    if (input.column_partials && partial_rows) {
+        *partial_rows = int(first.grid);
+    }
+    launch_chained(kernel, first.grid + second.grid, kThreads,
+                   std::max(first.smem_bytes, second.smem_bytes), stream, first.maps,
+                   second.maps, first.p, second.p, int(first.grid));
+    ++g_kernel_launches;
+    g_tc_products += 2;
     return 0;
 }
 

@@ -42,6 +42,11 @@ bool gemm_tc_supported(const TcGemm &gemm);
 // *partial_rows receives the number of rows of column_partials written.
 int launch_gemm_tc(const TcGemm &gemm, cudaStream_t stream,
                    int *partial_rows = nullptr);
+// The two gradients of a linear layer [m,k] x [k,n] in one launch, when both are small
+// enough to run side by side (gemm_tc_pairs).  -1, with nothing launched, otherwise.
+bool gemm_tc_pairs(int m, int k, int n);
+int launch_gemm_tc_pair(const TcGemm &input, const TcGemm &weight, cudaStream_t stream,
+                        int *partial_rows = nullptr);
 // 0, or the code of the first bounded wait that expired inside the kernel.
 int gemm_tc_status();
 // Products launched on the tensor cores since the library was loaded, and

@@ -359,5 +359,10 @@ bool launch_gemm_thin(const FmaGemm &gemm, cudaStream_t stream);
 // *partial_rows receives the number of rows of column_partials written.
 int launch_gemm_fma(const FmaGemm &gemm, cudaStream_t stream,
                     int *partial_rows = nullptr);
+// The two gradients of a linear layer [m,k] x [k,n] in one launch, when both run on
+// the smallest tile (gemm_fma_pairs).  -1, with nothing launched, otherwise.
+bool gemm_fma_pairs(int m, int k, int n);
+int launch_gemm_fma_pair(const FmaGemm &input, const FmaGemm &weight, cudaStream_t stream,
+                         int *partial_rows);
 
 }  // namespace vitb200
