@@ -289,6 +289,15 @@ def test_attention_forward_and_backward(lib, groups, seq, hd, precision):
     np.testing.assert_allclose(host(tp).sum(axis=1), 1.0, atol=1e-5)
 
 
+@pytest.mark.parametrize("groups,seq,hd", [
+    (1, 129, 1), (2, 191, 8), (1, 192, 10), (3, 193, 16), (2, 130, 33), (1, 256, 100),
+    (2, 200, 128)])
+def test_long_fp32_attention_at_the_edges_of_its_tiles(lib, groups, seq, hd):
+    """64 x 64 tiles with one row, one short of a row and a whole row left over; head
+    dimensions below, at and between the kernels', with and without 16-byte rows."""
+    test_attention_forward_and_backward(lib, groups, seq, hd, FP32)
+
+
 @pytest.mark.parametrize("precision", [FP32, TF32], ids=["fp32", "tf32"])
 @pytest.mark.parametrize("groups,seq,hd", [
     (1, 1, 16), (3, 5, 16), (16, 50, 16), (5, 64, 16), (4, 17, 32),
