@@ -16,7 +16,9 @@
 // contracted index outermost in shared memory, so that 16 multiply-adds cost two
 // 128-bit reads.  A thread's four keys of a tile are 16 apart (their operand is
 // staged in that order), so that its accesses to rows of P are contiguous across
-// lanes.  MEASURED
+// lanes.  Measured against 32 x 32 tiles with scalar reads, us forward / backward:
+// 153 groups of 442 x 32 608 / 1415 -> 254 / 423, 40 of 1025 x 64 1595 / 3727 -> 671 /
+// 1167 (23 TFLOP/s, recomputed scores counted), 6 of 170 x 8 18 / 45 -> 18 / 30.
 #include "kernels.h"
 #include "gemm.h"
 #include "../../include/vitb200.h"
