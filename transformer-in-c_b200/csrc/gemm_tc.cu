@@ -16,7 +16,7 @@
 // of the reduction); three warp roles meet only through mbarriers:
 //
 //   warp 0      TMA producer: per 32-deep reduction block, one 128B-swizzled
-//               box (K-major) or four 32x32 boxes (MN-major) per operand into
+//               box (K-major) or a box of 32x32 blocks (MN-major) per operand into
 //               a shared-memory ring of 32 KB stages (2 stages by default)
 //   warp 1      allocates 256 TMEM columns (two accumulators), issues four
 //               K=8 tcgen05.mma per block from one lane, releases stages with
@@ -74,6 +74,7 @@ struct TcParams {
     int staging_bytes;        // epilogue staging: 16 or 32 KiB
     int m_tiles, n_tiles;
     int a_mn_major, b_mn_major;
+    int a_blocked, b_blocked; // MN-major operand: one copy per tile (see operand_map)
     int reduce_add;           // 1: TMA reduce-add into D, 0: plain store
     const float *bias;        // nullable, length n
     const float *residual;    // [m, n] with residual_pitch, for kSecondResidual
@@ -214,7 +215,9 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
                     uint8_t *b_tile = a_tile + kABytes;
                     const int k0 = kb * kBlockK;
                     mbarrier_expect_tx(&full_bar[s], kStageBytes);
-                    if (p.a_mn_major) {
+                    if (p.a_blocked) {
+                        tma_load_3d(a_tile, &map_a, 0, k0, m0 / 32, &full_bar[s]);
+                    } else if (p.a_mn_major) {
                         for (int j = 0; j < TILE_M / 32; ++j) {
                             tma_load_2d(a_tile + j * 4096, &map_a, m0 + 32 * j, k0,
                                         &full_bar[s]);
@@ -223,7 +226,9 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
                         // One box of TILE_M rows (the map's box height).
                         tma_load_2d(a_tile, &map_a, k0, m0, &full_bar[s]);
                     }
-                    if (p.b_mn_major) {
+                    if (p.b_blocked) {
+                        tma_load_3d(b_tile, &map_b, 0, k0, n0 / 32, &full_bar[s]);
+                    } else if (p.b_mn_major) {
                         for (int j = 0; j < TILE_N / 32; ++j) {
                             tma_load_2d(b_tile + j * 4096, &map_b, n0 + 32 * j, k0,
                                         &full_bar[s]);
@@ -719,12 +724,13 @@ EncodeTiled encode_tiled() {
 struct MapKey {
     const void *base;
     unsigned long long inner, outer, pitch;
-    unsigned box_inner, box_outer;
+    unsigned box_inner, box_outer, blocks;
     int swizzle;
     bool operator==(const MapKey &o) const {
         return base == o.base && inner == o.inner && outer == o.outer &&
                pitch == o.pitch && box_inner == o.box_inner &&
-               box_outer == o.box_outer && swizzle == o.swizzle;
+               box_outer == o.box_outer && blocks == o.blocks &&
+               swizzle == o.swizzle;
     }
 };
 
@@ -735,7 +741,7 @@ struct MapKeyHash {
         h = h * 1000003u ^ k.outer;
         h = h * 1000003u ^ k.pitch;
         h = h * 1000003u ^ (size_t(k.box_inner) << 16 | k.box_outer);
-        h = h * 1000003u ^ size_t(k.swizzle);
+        h = h * 1000003u ^ (size_t(k.swizzle) << 16 | k.blocks);
         return h;
     }
 };
@@ -745,14 +751,17 @@ struct MapKeyHash {
 // flavour.  Operand maps use the TFLOAT32 element type, which makes the copy
 // engine round the FP32 words to TF32 (nearest) on their way into shared
 // memory instead of leaving the truncation to the MMA; the output map is plain
-// FP32.  Encoded maps are cached: the training step presents the same buffers
-// every iteration.
+// FP32.  blocks > 0: the row is cut into blocks of box_inner elements (it must be a
+// multiple of them) and a copy takes that many blocks of box_outer rows each, one
+// after the other, from coordinates (0, row, block) on.  Encoded maps are cached: the
+// training step presents the same buffers every iteration.
 bool tensor_map(const float *base, unsigned long long inner,
                 unsigned long long outer, unsigned long long pitch,
                 unsigned box_inner, unsigned box_outer,
-                CUtensorMapSwizzle swizzle, bool as_tf32, CUtensorMap *out) {
+                CUtensorMapSwizzle swizzle, bool as_tf32, CUtensorMap *out,
+                unsigned blocks = 0) {
     static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
-    const MapKey key{base, inner, outer, pitch, box_inner, box_outer,
+    const MapKey key{base, inner, outer, pitch, box_inner, box_outer, blocks,
                      int(swizzle) * 2 + int(as_tf32)};
     auto found = cache.find(key);
     if (found != cache.end()) {
@@ -763,13 +772,14 @@ bool tensor_map(const float *base, unsigned long long inner,
     if (!encode) {
         return false;
     }
-    const cuuint64_t dims[2] = {inner, outer};
-    const cuuint64_t strides[1] = {pitch * sizeof(float)};
-    const cuuint32_t box[2] = {box_inner, box_outer};
-    const cuuint32_t element_strides[2] = {1, 1};
+    const cuuint64_t dims[3] = {blocks ? box_inner : inner, outer, inner / box_inner};
+    const cuuint64_t strides[2] = {pitch * sizeof(float), box_inner * sizeof(float)};
+    const cuuint32_t box[3] = {box_inner, box_outer, blocks};
+    const cuuint32_t element_strides[3] = {1, 1, 1};
     const CUresult status = encode(
         out, as_tf32 ? CU_TENSOR_MAP_DATA_TYPE_TFLOAT32
-                     : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims,
+                     : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+        blocks ? 3 : 2, const_cast<float *>(base), dims,
         strides, box, element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
         swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -781,6 +791,18 @@ bool tensor_map(const float *base, unsigned long long inner,
     }
     cache.emplace(key, *out);
     return true;
+}
+
+// MN-major operand: rows = reduction index, inner = output index, in 32 x 32 blocks.  A
+// tile is `blocks` of them in one copy where rows are whole blocks; otherwise a copy
+// each, whose columns past the row read as zero.  (One thread issues all copies, and
+// nine to sixteen for a block of the reduction keep it longer than the products keep
+// the tensor core: [65600,384]x[384,1152] 129 -> 109 us, weight gradient [1536,384]
+// over 65600 rows 151 -> 128, bias + GELU onto 2048 columns 129 -> 126.)
+bool operand_map(const float *base, unsigned long long inner, unsigned long long outer,
+                 unsigned long long pitch, unsigned blocks, CUtensorMap *out) {
+    return tensor_map(base, inner, outer, pitch, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B,
+                      true, out, blocks);
 }
 
 int *status_word() {
@@ -1000,14 +1022,14 @@ bool prepare(const TcGemm &g, int forced_narrow, long long most_ctas, TcLaunch *
     CUtensorMap &map_a = out->maps.a, &map_b = out->maps.b, &map_d = out->maps.d,
                 &map_d2 = out->maps.d2;
     // K-major operand: rows = output index, inner = reduction index.
-    // MN-major operand: rows = reduction index, inner = output index.
     const CUtensorMapSwizzle chunks16 = CU_TENSOR_MAP_SWIZZLE_128B;
-    const CUtensorMapSwizzle chunks32 = CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B;
+    const bool a_blocked = g.a_mn_major && g.m % 32 == 0;
+    const bool b_blocked = g.b_mn_major && g.n % 32 == 0;
     const bool ok_a = g.a_mn_major
-        ? tensor_map(g.a, g.m, g.k, g.lda, 32, 32, chunks32, true, &map_a)
+        ? operand_map(g.a, g.m, g.k, g.lda, a_blocked ? tile_m / 32 : 0, &map_a)
         : tensor_map(g.a, g.k, g.m, g.lda, 32, tile_m, chunks16, true, &map_a);
     const bool ok_b = g.b_mn_major
-        ? tensor_map(g.b, g.n, g.k, g.ldb, 32, 32, chunks32, true, &map_b)
+        ? operand_map(g.b, g.n, g.k, g.ldb, b_blocked ? tile_n / 32 : 0, &map_b)
         : tensor_map(g.b, g.k, g.n, g.ldb, 32, tile_n, chunks16, true, &map_b);
     const bool ok_d =
         tensor_map(g.d, g.n, g.m, g.ldd, 32, 32, chunks16, false, &map_d);
@@ -1103,6 +1125,8 @@ bool prepare(const TcGemm &g, int forced_narrow, long long most_ctas, TcLaunch *
     splits = (p.k_blocks + p.k_blocks_per_split - 1) / p.k_blocks_per_split;
     p.a_mn_major = g.a_mn_major ? 1 : 0;
     p.b_mn_major = g.b_mn_major ? 1 : 0;
+    p.a_blocked = a_blocked ? 1 : 0;
+    p.b_blocked = b_blocked ? 1 : 0;
     p.reduce_add = g.accumulate ? 1 : 0;
     p.bias = g.bias;
     p.column_partials = g.column_partials;
