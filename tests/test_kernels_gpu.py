@@ -79,6 +79,54 @@ def test_gemm_fp32_forward_and_backward(lib, m, k, n):
 
 
 @pytest.mark.parametrize("m,k,n", [
+    (12800, 128, 128), (12833, 100, 132), (9000, 256, 384), (19000, 36, 260)])
+def test_large_fp32_products_keep_the_precision_of_fp32(lib, m, k, n):
+    """Products whose operands are split for the tensor cores: whole tiles, and rows,
+    columns and reductions with remainders of them.  2-norm error against 64 bits: a sum
+    has one rounding (6e-8 at most, 2.5e-8 rms) per 64 terms and four truncated additions
+    (6e-8 on average) between two of them; a weight gradient up to 37 slices more.  One
+    chain of FMAs has 2.0e-7 at 128 terms and would fail."""
+    rng = np.random.RandomState(m)
+    x, w, dy = (rng.randn(*shape).astype(np.float32) for shape in ((m, k), (k, n), (m, n)))
+    tx, tw, tdy, ty = dev(x), dev(w), dev(dy), torch.empty(m, n, device="cuda")
+    tdx, tdw = torch.zeros(m, k, device="cuda"), torch.zeros(k, n, device="cuda")
+    sizes = (size(m), size(k), size(n), FP32, None)
+    assert lib.vitb200_k_gemm(ptr(tx), ptr(tw), ptr(ty), *sizes) == 0
+    assert lib.vitb200_k_gemm_backward(ptr(tx), ptr(tw), ptr(tdy), ptr(tdx), ptr(tdw),
+                                       *sizes) == 0
+    x, w, dy = (a.astype(np.float64) for a in (x, w, dy))
+    for got, want, bound in ((ty, x @ w, 1.3e-7), (tdx, dy @ w.T, 1.3e-7),
+                             (tdw, x.T @ dy, 2.5e-7)):
+        error = np.linalg.norm(host(got) - want) / np.linalg.norm(want)
+        assert error <= bound, (error, bound)
+
+
+def test_large_fp32_products_of_infinities(lib):
+    """What has no finite parts gives what FMAs give: infinities of the right sign, not a
+    number where they meet or where one was, and finite sums of the largest values."""
+    m, k, n = 12800, 128, 128
+    rng = np.random.RandomState(5)
+    x, w = rng.randn(m, k).astype(np.float32), rng.randn(k, n).astype(np.float32)
+    x[3, 7] = np.inf
+    x[130, 0] = -np.inf
+    x[131, 5], x[131, 6] = np.inf, -np.inf
+    x[5000, 127] = np.nan
+    x[12799] = 0.0
+    x[12799, 64] = np.finfo(np.float32).max
+    w[64] = 0.5
+    tx, tw, ty = dev(x), dev(w), torch.empty(m, n, device="cuda")
+    assert lib.vitb200_k_gemm(ptr(tx), ptr(tw), ptr(ty), size(m), size(k), size(n), FP32,
+                              None) == 0
+    got = host(ty)
+    with np.errstate(invalid="ignore"):
+        want = x.astype(np.float64) @ w.astype(np.float64)
+    for row in (3, 130, 131, 5000, 12799):
+        assert np.array_equal(got[row], want[row].astype(np.float32), equal_nan=True), row
+    rest = np.delete(np.arange(m), (3, 130, 131, 5000, 12799))
+    close(got[rest], want[rest], 1e-5)
+
+
+@pytest.mark.parametrize("m,k,n", [
     (128, 32, 128), (128, 128, 128), (200, 96, 160), (1600, 128, 384),
     (1000, 512, 128), (4096, 128, 512), (333, 36, 44), (102400, 128, 128),
     (257, 1024, 256), (1568, 16, 128), (300, 16, 48), (100, 48, 16),

@@ -657,7 +657,23 @@ struct FmaLaunch {
     int tile, slices;
 };
 
-bool prepare(const FmaGemm &g, cudaStream_t stream, int *partial_rows, FmaLaunch *out) {
+Form form_of(const FmaGemm &g) {
+    return g.a_k ? (g.b_k ? Form::InputGradient : Form::Forward) : Form::WeightGradient;
+}
+
+// K slices may only add into C.
+bool adds_to_c(const FmaGemm &g) {
+    return g.accumulate && form_of(g) != Form::Forward;
+}
+
+FmaPlan plan_of(const FmaGemm &g) {
+    return adds_to_c(g)
+        ? plan_addition(g.m, g.n, g.k, form_of(g) == Form::InputGradient)
+        : plan_product(g.m, g.n, g.k, false, true, LLONG_MAX);
+}
+
+bool prepare(const FmaGemm &g, const FmaPlan &plan, cudaStream_t stream, int *partial_rows,
+             FmaLaunch *out) {
     FmaParams &p = out->p;
     p = FmaParams{};
     p.a = g.a;
@@ -678,16 +694,11 @@ bool prepare(const FmaGemm &g, cudaStream_t stream, int *partial_rows, FmaLaunch
               (!g.gelu_out || aligned16(g.gelu_out)) &&
               (!g.gelu_input || aligned16(g.gelu_input));
     p.accumulate = g.accumulate ? 1 : 0;
-    const Form form = g.a_k ? (g.b_k ? Form::InputGradient : Form::Forward)
-                            : Form::WeightGradient;
+    const Form form = form_of(g);
     if (form == Form::WeightGradient && (!g.accumulate || g.b_k)) {
         return false;   // no caller has this form
     }
-    // K slices may only add into C.
-    const bool adds = g.accumulate && form != Form::Forward;
-    const FmaPlan plan = adds
-        ? plan_addition(g.m, g.n, g.k, form == Form::InputGradient)
-        : plan_product(g.m, g.n, g.k, false, true, LLONG_MAX);
+    const bool adds = adds_to_c(g);
     int slices = plan.slices;
     p.k_per_split = slice_length(g.k, slices);
     if (adds && !plan.cluster && slices > 1) {
@@ -722,8 +733,15 @@ int launch_gemm_fma(const FmaGemm &g, cudaStream_t stream, int *partial_rows) {
         ++g_fma_products;
         return 0;
     }
+    // (Slices in a cluster keep sums of positive terms closer than anything else does.)
+    const FmaPlan plan = plan_of(g);
+    if (!(plan.cluster && plan.slices > 1) && gemm_split_clocks(g) < plan.clocks &&
+        launch_gemm_split(g, stream, partial_rows)) {
+        ++g_fma_products;
+        return 0;
+    }
     FmaLaunch launch;
-    if (!prepare(g, stream, partial_rows, &launch)) {
+    if (!prepare(g, plan, stream, partial_rows, &launch)) {
         return -1;
     }
     const FmaParams &p = launch.p;
@@ -768,8 +786,8 @@ int launch_gemm_fma_pair(const FmaGemm &input, const FmaGemm &weight, cudaStream
                          int *partial_rows) {
     FmaLaunch first, second;
     if (input.accumulate || !gemm_fma_pairs(input.m, input.n, input.k) ||
-        !prepare(input, stream, partial_rows, &first) ||
-        !prepare(weight, stream, nullptr, &second) ||
+        !prepare(input, plan_of(input), stream, partial_rows, &first) ||
+        !prepare(weight, plan_of(weight), stream, nullptr, &second) ||
         first.form != Form::InputGradient || second.form != Form::WeightGradient ||
         first.tile != kSmallestTile || second.tile != kSmallestTile) {
         return -1;

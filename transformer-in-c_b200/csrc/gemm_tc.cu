@@ -1252,6 +1252,14 @@ int launch_gemm_tc_pair(const TcGemm &input, const TcGemm &weight, cudaStream_t 
     return 0;
 }
 
+bool gemm_plain_map(const float *base, unsigned long long inner, unsigned long long outer,
+                    unsigned long long pitch, unsigned box_inner, unsigned box_outer,
+                    bool swizzled, CUtensorMap *out) {
+    return tensor_map(base, inner, outer, pitch, box_inner, box_outer,
+                      swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                      false, out);
+}
+
 unsigned long long g_tc_products = 0, g_tc_wide_products = 0;
 
 int gemm_tc_status() {

@@ -1,6 +1,7 @@
 // tcgen05 / TMA matrix product (gemm_tc.cu).
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 namespace vitb200 {
@@ -52,6 +53,11 @@ int gemm_tc_status();
 // Products launched on the tensor cores since the library was loaded, and
 // how many of them used the 128 x 256 tile.
 extern unsigned long long g_tc_products, g_tc_wide_products;
+// Tensor map of an FP32 matrix (`outer` rows of `inner` contiguous floats, `pitch` apart)
+// in plain boxes, or with 128-byte rows in the 128-byte swizzle.
+bool gemm_plain_map(const float *base, unsigned long long inner, unsigned long long outer,
+                    unsigned long long pitch, unsigned box_inner, unsigned box_outer,
+                    bool swizzled, CUtensorMap *out);
 // Device address of that status word, shared by every kernel of the library
 // that waits on an mbarrier (codes 1..15: matrix product, 16..: attention);
 // nullptr when it could not be mapped.
