@@ -735,7 +735,8 @@ int launch_gemm_fma(const FmaGemm &g, cudaStream_t stream, int *partial_rows) {
     }
     // (Slices in a cluster keep sums of positive terms closer than anything else does.)
     const FmaPlan plan = plan_of(g);
-    if (!(plan.cluster && plan.slices > 1) && gemm_split_clocks(g) < plan.clocks &&
+    if (plan.clocks > 15000.0 && !(plan.cluster && plan.slices > 1) &&
+        gemm_split_clocks(g) < plan.clocks &&
         launch_gemm_split(g, stream, partial_rows)) {
         ++g_fma_products;
         return 0;
