@@ -61,7 +61,14 @@ constexpr int kThreads = 192;
 // The tall tile has a group of four epilogue warps for each of its two
 // accumulators, so that both drain at the same time.
 constexpr int kThreadsTall = 320;
-constexpr int kBarrierBytes = 256;   // 2 x kMaxStages + 4 + 8 mbarriers, TMEM slot
+// So do the GELU's two epilogues on the tiles that large products run on, whose warps
+// wait for memory between their arithmetic: more of them wait at a time.
+template <int TILE_M, int TILE_N, int SECOND>
+constexpr bool kTwoGroups =
+    TILE_M == 256 || (TILE_N == 256 && (SECOND == 1 || SECOND == 3)) || SECOND == 4;
+template <int TILE_M, int TILE_N, int SECOND>
+constexpr int kThreadsOf = kTwoGroups<TILE_M, TILE_N, SECOND> ? kThreadsTall : kThreads;
+constexpr int kBarrierBytes = 320;   // 2 x kMaxStages + 4 + 16 mbarriers, TMEM slot
 
 using namespace tc;
 
@@ -90,6 +97,10 @@ constexpr int kSecondResidual = 2;   // D = A*B + bias, D2 = D + residual
 // map_d2 (one 32 x 32 block per accumulator block, by TMA into the block the
 // result is then staged in); there is one output.
 constexpr int kGeluSlope = 3;
+// The same with eight epilogue warps of one staging block each on the square tile.
+constexpr int kGeluSlopeEight = 4;
+template <int SECOND>
+constexpr bool kIsSlope = SECOND == kGeluSlope || SECOND == kGeluSlopeEight;
 
 // Persistent kernel: each CTA walks work items (output tile x reduction
 // slice) item = cta, cta + ctas, ...; the three roles run
@@ -136,7 +147,7 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
     uint64_t *tmem_full_bar = empty_bar + kMaxStages;
     uint64_t *tmem_empty_bar = tmem_full_bar + 2;
     uint32_t &tmem_base_slot = *reinterpret_cast<uint32_t *>(tmem_empty_bar + 2);
-    uint64_t *operand_bar = tmem_empty_bar + 3;   // two per epilogue warp
+    uint64_t *operand_bar = tmem_empty_bar + 3;   // up to two per epilogue warp
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     if ((smem_address(smem) & 1023u) != 0) {
@@ -155,9 +166,11 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
         }
         for (int b = 0; b < 2; ++b) {
             mbarrier_init(&tmem_full_bar[b], 1);
-            mbarrier_init(&tmem_empty_bar[b], 4);   // one arrival per epilogue warp
+            // One arrival per epilogue warp that reads the accumulator.
+            mbarrier_init(&tmem_empty_bar[b],
+                          kHalves == 1 && kTwoGroups<TILE_M, TILE_N, SECOND> ? 8 : 4);
         }
-        for (int w = 0; w < 8; ++w) {
+        for (int w = 0; w < 16; ++w) {
             mbarrier_init(&operand_bar[w], 1);
         }
         prefetch_tensor_map(&map_a);
@@ -182,7 +195,7 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
     // touched, so the kernel before this one in the stream has to be complete.
     grid_dependency_wait();
     grid_dependency_release();
-    if (SECOND == kGeluSlope && p.column_partials) {
+    if (kIsSlope<SECOND> && p.column_partials) {
         // This CTA's own row of column sums, which its epilogue warps add into.
         for (int c = threadIdx.x; c < p.n; c += blockDim.x) {
             p.column_partials[size_t(cta) * p.n + c] = 0.0f;
@@ -324,16 +337,19 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
                 }
             }
         }
-    } else if constexpr (SECOND == kGeluSlope) {
-        // Epilogue of D = (A*B) * gelu'(H).  Each warp walks its 32 x 32
-        // blocks in order (tile after tile, four column chunks per tile) as a
-        // two-deep pipeline over its two staging blocks: while block j is
-        // multiplied and stored, the copy engine already fetches the H values
-        // of block j+1 into the other staging block, so the latency of that
-        // read stays off the critical path.
+    } else if constexpr (kIsSlope<SECOND>) {
+        // Epilogue of D = (A*B) * gelu'(H).  Each warp walks its 32 x 32 blocks in order
+        // (tile after tile, its column chunks of each).  The H values of a block are
+        // fetched by the copy engine into the staging block that the result then leaves
+        // from: with two staging blocks the ones of block j+1 while block j is
+        // multiplied, with one as soon as the result of block j has been read.
+        constexpr int kGroups = kTwoGroups<TILE_M, TILE_N, SECOND> ? 2 : 1;
+        constexpr int kBlocks = SECOND == kGeluSlopeEight ? 1 : 2;
+        constexpr int kChunks = TILE_N / 32 / kGroups;   // of a warp and tile
         const int quarter = warp & 3;
-        uint8_t *my_staging = staging + quarter * (p.staging_bytes / 4);
-        uint64_t *my_bar = operand_bar + 2 * quarter;
+        const int first_chunk = kGroups == 2 ? (warp - 2) / 4 * kChunks : 0;
+        uint8_t *my_staging = staging + (warp - 2) * kBlocks * 4096;
+        uint64_t *my_bar = operand_bar + (warp - 2) * kBlocks;
         uint32_t phases = 0;   // bit b: parity of the next completion of my_bar[b]
         int issued = 0;        // H blocks requested so far
         int consumed = 0;      // H blocks used so far
@@ -347,17 +363,25 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
             }
             if (lane == 0) {
                 // The block was last read by the store issued for the block
-                // before the current one.
+                // before the current one (kBlocks == 1: for the current one).
                 asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                const int b = issued & 1;
+                const int b = issued % kBlocks;
                 mbarrier_expect_tx(&my_bar[b], 4096);
                 tma_load_2d(my_staging + b * 4096, &map_d2, col0, m0, &my_bar[b]);
             }
             ++issued;
         };
+        // The block after (item, chunk), possibly the next tile's first.
+        auto request_after = [&](int item, int chunk) {
+            if (chunk + 1 < first_chunk + kChunks) {
+                request(item, chunk + 1);
+            } else if (item + ctas < items) {
+                request(item + ctas, first_chunk);
+            }
+        };
         if (cta < items) {
-            request(cta, 0);
+            request(cta, first_chunk);
         }
         int local = 0;
         for (int item = cta; item < items && ok; item += ctas, ++local) {
@@ -374,7 +398,7 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
             }
             tcgen05_fence_after();
 #pragma unroll 1
-            for (int chunk = 0; chunk < TILE_N / 32; ++chunk) {
+            for (int chunk = first_chunk; chunk < first_chunk + kChunks; ++chunk) {
                 const int col0 = n0 + chunk * 32;
                 const bool chunk_live = col0 < p.n && m0 < p.m;
                 uint32_t r[32];
@@ -383,23 +407,20 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
                                         buffer * TILE_N + chunk * 32,
                                     r);
                 }
-                if (chunk == TILE_N / 32 - 1) {
+                if (chunk == first_chunk + kChunks - 1) {
                     tcgen05_fence_before();
                     __syncwarp();
                     if (lane == 0) {
                         mbarrier_arrive(&tmem_empty_bar[buffer]);
                     }
                 }
-                // The block after this one, possibly the next tile's first.
-                if (chunk + 1 < TILE_N / 32) {
-                    request(item, chunk + 1);
-                } else if (item + ctas < items) {
-                    request(item + ctas, 0);
+                if (kBlocks == 2 || !chunk_live) {
+                    request_after(item, chunk);
                 }
                 if (!chunk_live) {
                     continue;   // uniform across the warp
                 }
-                const int b = consumed & 1;
+                const int b = consumed % kBlocks;
                 ++consumed;
                 ok = mbarrier_wait(&my_bar[b], (phases >> b) & 1u);
                 ok = __all_sync(0xffffffffu, ok);
@@ -443,6 +464,9 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
                     tma_store_2d(block, &map_d, col0, m0);
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
+                if (kBlocks == 1) {
+                    request_after(item, chunk);
+                }
             }
         }
         if (lane == 0) {
@@ -460,10 +484,14 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
         // given the space instead.
         // The tall tile: warps 2-5 drain the upper half's accumulator, warps
         // 6-9 the lower half's, each warp through one 4 KiB block.
+        // Two groups on one accumulator take half of its columns each.
+        constexpr bool kEight = kTwoGroups<TILE_M, TILE_N, SECOND>;
+        constexpr int kChunks = TILE_N / 32 / (kEight && kHalves == 1 ? 2 : 1);
         const int half = kHalves == 2 ? (warp - 2) >> 2 : 0;
+        const int first_chunk = kEight && kHalves == 1 ? (warp - 2) / 4 * kChunks : 0;
         const int buffers =
-            kHalves == 2 ? 1 : (outputs == 2 ? 1 : p.staging_bytes / (4 * 4096));
-        uint8_t *my_staging = kHalves == 2
+            kEight ? 1 : (outputs == 2 ? 1 : p.staging_bytes / (4 * 4096));
+        uint8_t *my_staging = kEight
             ? staging + (warp - 2) * 4096
             : staging + quarter * (p.staging_bytes / 4);
         int local = 0;
@@ -483,7 +511,7 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
             }
             tcgen05_fence_after();
 #pragma unroll 1
-            for (int chunk = 0; chunk < TILE_N / 32; ++chunk) {
+            for (int chunk = first_chunk; chunk < first_chunk + kChunks; ++chunk) {
                 const int col0 = n0 + chunk * 32;
                 const bool chunk_live = col0 < p.n && m0 < p.m;
                 // Bias for these 32 columns, requested before the accumulator
@@ -510,7 +538,7 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
                                         buffer * TILE_N + chunk * 32,
                                     r);
                 }
-                if (chunk == TILE_N / 32 - 1) {
+                if (chunk == first_chunk + kChunks - 1) {
                     // Everything this warp needs is in registers: hand the
                     // accumulator buffer back to the MMA warp.
                     tcgen05_fence_before();
@@ -549,7 +577,7 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
                 // With 16 KiB of staging both outputs of a warp go through the
                 // same 4 KiB block, one after the other.
                 const bool shared_block =
-                    outputs == 2 && (kHalves == 2 || p.staging_bytes == kOperandBytes);
+                    outputs == 2 && (kEight || p.staging_bytes == kOperandBytes);
                 float *second = shared_block
                     ? first : reinterpret_cast<float *>(my_staging + 4096);
                 {
@@ -668,7 +696,7 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
 }
 
 template <int TILE_M, int TILE_N, int SECOND>
-__global__ void __launch_bounds__(TILE_M == 2 * kTileM ? kThreadsTall : kThreads)
+__global__ void __launch_bounds__(kThreadsOf<TILE_M, TILE_N, SECOND>)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
                const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_d,
@@ -826,27 +854,33 @@ using TcKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMa
 // tile's would write out of range: so kernels are named here, beside their extents,
 // and nowhere else.
 struct TcTile {
-    int m, n, threads;
-    TcKernel plain, second_gelu, second_residual, gelu_slope;   // null: not built
+    int m, n;
+    // (Null: not built.)
+    TcKernel plain, second_gelu, second_residual, gelu_slope, gelu_slope_eight;
+    int threads[5];
 
     TcKernel kernel(int second) const {
         return second == kSecondGelu       ? second_gelu
                : second == kSecondResidual ? second_residual
                : second == kGeluSlope      ? gelu_slope
+               : second == kGeluSlopeEight ? gelu_slope_eight
                                            : plain;
     }
 };
 
 template <int M, int N>
 constexpr TcTile make_tile() {
-    TcTile tile = {M, N, M == 2 * kTileM ? kThreadsTall : kThreads,
-                   gemm_tc_kernel<M, N, 0>, gemm_tc_kernel<M, N, kSecondGelu>,
-                   nullptr, nullptr};
-    if constexpr (M == kTileM && N <= kTileN) {
+    TcTile tile = {M, N, gemm_tc_kernel<M, N, 0>, gemm_tc_kernel<M, N, kSecondGelu>,
+                   nullptr, nullptr, nullptr,
+                   {kThreadsOf<M, N, 0>, kThreadsOf<M, N, kSecondGelu>,
+                    kThreadsOf<M, N, kSecondResidual>, kThreadsOf<M, N, kGeluSlope>,
+                    kThreadsOf<M, N, kGeluSlopeEight>}};
+    if constexpr (M == kTileM) {
         tile.gelu_slope = gemm_tc_kernel<M, N, kGeluSlope>;
     }
     if constexpr (M == kTileM && N == kTileN) {
         tile.second_residual = gemm_tc_kernel<M, N, kSecondResidual>;
+        tile.gelu_slope_eight = gemm_tc_kernel<M, N, kGeluSlopeEight>;
     }
     return tile;
 }
@@ -859,11 +893,11 @@ const TcTile kTcTiles[kTcTileCount] = {
 // Lets every kernel use the whole of an SM's shared memory.
 bool raise_limits() {
     static SharedMemoryLimit limit;
-    const void *kernels[4 * kTcTileCount];
+    const void *kernels[5 * kTcTileCount];
     int count = 0;
     for (const TcTile &tile : kTcTiles) {
         for (TcKernel kernel : {tile.plain, tile.second_gelu, tile.second_residual,
-                                tile.gelu_slope}) {
+                                tile.gelu_slope, tile.gelu_slope_eight}) {
             if (kernel) {
                 kernels[count++] = reinterpret_cast<const void *>(kernel);
             }
@@ -955,10 +989,10 @@ bool prepare(const TcGemm &g, int forced_narrow, long long most_ctas, TcLaunch *
     const bool divides = g.n % 256 == 0 ||
                          (g.n % 128 == 0 && g.n >= 256 &&
                           (g.n >= 1024 || (!g.accumulate && g.k >= 1024)));
-    bool wide = (!g.d2 || gelu_pair) && !g.gelu_input && g.k >= 256 && divides;
-    if (forced_tile == 128 || (g.d2 && !gelu_pair) || g.gelu_input) {
+    bool wide = (!g.d2 || gelu_pair) && g.k >= (g.gelu_input ? 512 : 256) && divides;
+    if (forced_tile == 128 || (g.d2 && !gelu_pair)) {
         wide = false;
-    } else if (forced_tile == 256 && !g.d2) {
+    } else if (forced_tile == 256 && !g.d2 && !g.gelu_input) {
         wide = g.n >= 256;
     }
     // Tall tiles (256 x 256, two accumulator halves) on top of that when there
@@ -972,13 +1006,14 @@ bool prepare(const TcGemm &g, int forced_narrow, long long most_ctas, TcLaunch *
     // is a small share of the rows.
     const bool fits = g.m % (2 * kTileM) == 0 || g.m % (2 * kTileM) > kTileM ||
                       g.m >= 16 * kTileM;
-    bool tall = wide && g.m >= 2 * kTileM && forced_tile_m != 128 &&
+    bool tall = wide && !g.gelu_input && g.m >= 2 * kTileM && forced_tile_m != 128 &&
                 ((long_enough && fits) || forced_tile_m == 256);
     // The GELU pair's epilogue (two stores and a GELU per element) takes
     // longer than the tile's products: the tall tile, whose accumulators are
     // not double-buffered across tiles, leaves it exposed; the 128 x 256 tile
     // hides the next tile's products behind it (measured 3 to 10 % faster at
-    // [100864,512]x[512,2048] and [65600,384]x[384,1536]).
+    // [100864,512]x[512,2048] and [65600,384]x[384,1536]).  Eight epilogue warps on it
+    // instead of four: 202 -> 196 us at the latter, 126 -> 124 at [25216,512]x[512,2048].
     static const bool gelu_pair_tall = getenv("VITB200_TC_GELU_TALL") != nullptr;
     if (gelu_pair && tall && !gelu_pair_tall) {
         tall = false;
@@ -1014,8 +1049,16 @@ bool prepare(const TcGemm &g, int forced_narrow, long long most_ctas, TcLaunch *
     const TcTile &tile =
         kTcTiles[narrow >= 0 ? narrow : (tall ? kTall : (wide ? kWide : kSquare))];
     const int tile_m = tile.m, tile_n = tile.n;
+    // The slope on square tiles: with a short reduction the epilogue outlasts the
+    // products, and eight warps get through it sooner (us, four warps -> eight: K = 128
+    // [102400,128]x[128,512] 90 -> 81, K = 256 [100864,256]x[256,1024] 193 -> 185); with
+    // a longer one they are in the way of the products' copies (K = 384 217 -> 233,
+    // K = 512 [25216,512]x[512,2048] 137 -> 149), and from 512 on the 128 x 256 tile is
+    // the faster (137 -> 132; 384: 217 -> 252).
+    const bool square = tile_m == kTileM && tile_n == kTileN;
     const int second = g.d2 ? (g.residual ? kSecondResidual : kSecondGelu)
-                            : (g.gelu_input ? kGeluSlope : 0);
+        : !g.gelu_input     ? 0
+        : square && g.k <= 256 ? kGeluSlopeEight : kGeluSlope;
     if (!tile.kernel(second)) {
         return false;
     }
@@ -1099,8 +1142,11 @@ bool prepare(const TcGemm &g, int forced_narrow, long long most_ctas, TcLaunch *
         const int depth = spread && !g.accumulate ? kMaxStages : 4;
         p.stages = std::max(2, std::min(depth, p.k_blocks));
     }
-    if (g.gelu_input) {
-        staging_bytes = 2 * kOperandBytes;   // its epilogue pipeline needs both blocks
+    if (g.gelu_input && tile_n > kTileN) {
+        staging_bytes = 4 * kOperandBytes;   // two blocks for each of eight warps
+        p.stages = 3;
+    } else if (g.gelu_input) {
+        staging_bytes = 2 * kOperandBytes;
         if (p.stages > 2 && ctas_per_sm > 1 && !narrowed) {
             p.stages = 2;
         }
@@ -1160,8 +1206,8 @@ int launch_gemm_tc(const TcGemm &g, cudaStream_t stream, int *partial_rows) {
         *partial_rows = int(launch.grid);
     }
     const TcPairMaps &maps = launch.maps;
-    launch_chained(launch.tile->kernel(launch.second), launch.grid, launch.tile->threads,
-                   launch.smem_bytes, stream, maps.a, maps.b, maps.d, maps.d2, launch.p);
+    launch_chained(launch.tile->kernel(launch.second), launch.grid,
+                   launch.tile->threads[launch.second], launch.smem_bytes, stream, maps.a, maps.b, maps.d, maps.d2, launch.p);
     ++g_kernel_launches;
     ++g_tc_products;
     if (launch.tile->n > kTileN) {
