@@ -467,3 +467,8 @@ def test_softmax_cross_entropy(lib, rows, cols, smoothing, weighted):
     # Existing gradient content is folded in before the division by rows
     # (reference src/ops.c:1063-1070).
     close(host(tg), grad0 / rows + grad, 1e-5)
+
+
+@pytest.mark.parametrize("rows,cols", [(33, 11), (128, 128), (128, 129), (129, 11)])
+def test_softmax_cross_entropy_in_one_block_and_in_two_kernels(lib, rows, cols):
+    test_softmax_cross_entropy(lib, rows, cols, 0.1, True)

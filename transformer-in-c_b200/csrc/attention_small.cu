@@ -207,6 +207,24 @@ __device__ __forceinline__ float lanes_max(float value) {
     return value;
 }
 
+// Adds one lane's COUNT values, over all rows of the block (the live ones), to the
+// column sums of its head; `columns` is in shared memory.
+template <int COUNT, int LANES>
+__device__ __forceinline__ void add_columns(float *columns, int part,
+                                            const float (&values)[COUNT], bool live) {
+#pragma unroll
+    for (int i = 0; i < COUNT; ++i) {
+        float sum = live ? values[i] : 0.0f;
+#pragma unroll
+        for (int distance = 16; distance >= LANES; distance /= 2) {
+            sum += __shfl_xor_sync(kFullMask, sum, distance);
+        }
+        if ((threadIdx.x & 31) < LANES) {
+            atomicAdd(columns + part * COUNT + i, sum);
+        }
+    }
+}
+
 // exp for softmax arguments (<= 0 after subtracting the row maximum):
 // ex2.approx on x * log2(e), relative error about 2e-7 in this range.
 __device__ __forceinline__ float softmax_exp(float x) {
@@ -325,7 +343,11 @@ attention_small_backward_kernel(
     float *__restrict__ dq, float *__restrict__ dk, float *__restrict__ dv,
     int seq, float scale, bool add_q, bool add_k, bool add_v, bool recompute,
     HeadLayout in_layout, HeadLayout out_layout, HeadLayout dout_layout,
-    HeadLayout grad_layout) {
+    HeadLayout grad_layout, float *__restrict__ column_partials) {
+    // Column sums of this head's dQ, dK and dV, where they are wanted: the QKV bias
+    // gradient then reads one row per sample instead of the whole projected gradient
+    // in a launch of its own.
+    __shared__ float columns[3 * HD];
     extern __shared__ __align__(16) float shared[];
     constexpr int kPitch = kTilePitch<HD>;
     constexpr bool kTwoTiles = HD < 64 && LANES > 1;   // P and dS side by side,
@@ -342,6 +364,9 @@ attention_small_backward_kernel(
     const int part = threadIdx.x % LANES;
     const bool live = threadIdx.x / LANES < seq;
     const int row = min(int(threadIdx.x) / LANES, seq - 1);
+    for (int c = threadIdx.x; c < 3 * HD; c += blockDim.x) {
+        columns[c] = 0.0f;
+    }
     grid_dependency_wait();
     grid_dependency_release();
     load_rows<HD>(q + base, q_tile, seq, in_layout.ld);
@@ -401,6 +426,9 @@ attention_small_backward_kernel(
         if (live) {
             store_part<HD / LANES>(dv + grad_row, part, sums, add_v);
         }
+        if (column_partials) {
+            add_columns<HD / LANES, LANES>(columns + 2 * HD, part, sums, live);
+        }
         __syncthreads();
     }
     // Rows: score gradients, then dQ_i.  (Every lane meets only its own keys.)
@@ -422,6 +450,9 @@ attention_small_backward_kernel(
         if (live) {
             store_part<HD / LANES>(dq + grad_row, part, sums, add_q);
         }
+        if (column_partials) {
+            add_columns<HD / LANES, LANES>(columns, part, sums, live);
+        }
     }
     __syncthreads();
     // Columns: dV_j (unless done), dK_j = sum_i dS_ij Q_i.
@@ -430,10 +461,26 @@ attention_small_backward_kernel(
         if (live) {
             store_part<HD / LANES>(dv + grad_row, part, sums, add_v);
         }
+        if (column_partials) {
+            add_columns<HD / LANES, LANES>(columns + 2 * HD, part, sums, live);
+        }
     }
     column(ds_tile, q_tile);
     if (live) {
         store_part<HD / LANES>(dk + grad_row, part, sums, add_k);
+    }
+    if (column_partials) {
+        add_columns<HD / LANES, LANES>(columns + HD, part, sums, live);
+    }
+    if (column_partials) {
+        // A row per sample: the columns of the projected gradient it belongs to.
+        __syncthreads();
+        const size_t heads = size_t(grad_layout.heads);
+        float *to = column_partials + group / heads * (3 * heads * HD) +
+                    group % heads * HD;
+        for (int c = threadIdx.x; c < 3 * HD; c += blockDim.x) {
+            to[c / HD * (heads * HD) + c % HD] = columns[c];
+        }
     }
 }
 
@@ -543,7 +590,8 @@ bool launch_attention_small_backward(const float *q, const float *k,
                                      cudaStream_t stream, HeadLayout in_layout,
                                      HeadLayout out_layout,
                                      HeadLayout dout_layout,
-                                     HeadLayout grad_layout) {
+                                     HeadLayout grad_layout,
+                                     float *column_partials) {
     in_layout = resolve_layout(in_layout, head_dim);
     out_layout = resolve_layout(out_layout, head_dim);
     dout_layout = resolve_layout(dout_layout, head_dim);
@@ -561,7 +609,7 @@ bool launch_attention_small_backward(const float *q, const float *k,
                            stream, q, k, v, probabilities, out, dout, dq, dk,  \
                            dv, int(seq), scale, add_q, add_k, add_v,           \
                            recompute, in_layout, out_layout, dout_layout,      \
-                           grad_layout) == cudaSuccess;                        \
+                           grad_layout, column_partials) == cudaSuccess;       \
     }
     VITB200_DISPATCH(head_dim, lanes, CALL)
 #undef CALL

@@ -18,6 +18,7 @@
 #include "data_parallel.h"
 #include "dataset.h"
 #include "gemm.h"
+#include "device_util.cuh"
 #include "gemm_tc.h"
 #include "kernels.h"
 
@@ -715,13 +716,13 @@ bool run_attention_backward(CudaBackend *backend,
             pending.out_layout, pending.dout_layout, grad_layout,
             column_partials);
     } else {
-        launch_attention_small_backward(
+        const bool launched = launch_attention_small_backward(
             pending.q, pending.k, pending.v, nullptr, pending.out,
             pending.dout, dq, dk, dv, groups, pending.seq, pending.head_dim,
             pending.scale, add_q, add_k, add_v, true, backend->stream,
             pending.in_layout, pending.out_layout, pending.dout_layout,
-            grad_layout);
-        partials_written = false;
+            grad_layout, column_partials);
+        partials_written = partials_written && launched;
     }
     return partials_written;
 }
@@ -1611,16 +1612,20 @@ int op_split_heads_backward(void *context, vitb200_tensor *projected,
         HeadLayout grad_layout;
         grad_layout.ld = int(3 * d_model);
         grad_layout.heads = int(heads);
-        // The tensor-core kernel also leaves per-sample column sums of what it
-        // writes: the QKV bias gradient the host asks for next
-        // (reference src/vit.c:588-591) then sums [batch, 3d] instead of
-        // [batch * seq, 3d].
+        // The kernel also leaves column sums of what it writes: the QKV bias
+        // gradient the host asks for next (reference src/vit.c:588-591) then sums
+        // [batch, 3d] instead of [batch * seq, 3d].
         // (Whole-group kernels: one row per sample.  tcgen05 kernels: one row
         // per CTA of their persistent grid.)
         const bool from_tc = pending.kind == 3 &&
                              tc_attention_wanted(seq, pending.head_dim);
+        // (The FP32 kernels only where a launch costs more than their sums, whose
+        // shuffles take longer than a pass over the gradient once two groups per SM
+        // are at work: FP32 batch 256 2820 -> 2845 us.)
+        const bool few_groups = batch * heads <= 2 * size_t(device_sm_count());
         const size_t partial_rows =
-            pending.kind == 2 ? batch : (from_tc ? attention_tc_partial_rows() : 0);
+            pending.kind == 2 || (pending.kind == 1 && few_groups)
+                ? batch : (from_tc ? attention_tc_partial_rows() : 0);
         float *partials = partial_rows
             ? partial_sums_buffer(backend, partial_rows * 3 * d_model)
             : nullptr;

@@ -256,6 +256,8 @@ bool launch_attention_tc_backward(const float *q, const float *k, const float *v
 // gradient; their column sums are the column sums of that gradient.
 size_t attention_tc_partial_rows();
 // recompute = true: `probabilities` is not read; P is rebuilt from Q and K.
+// column_partials (optional, grad_layout = {3 * d_model, heads}): a row of 3 * d_model
+// column sums of the projected gradient per sample.
 bool launch_attention_small_backward(const float *q, const float *k,
                                      const float *v, const float *probabilities,
                                      const float *out, const float *dout,
@@ -267,7 +269,8 @@ bool launch_attention_small_backward(const float *q, const float *k,
                                      HeadLayout in_layout = HeadLayout(),
                                      HeadLayout out_layout = HeadLayout(),
                                      HeadLayout dout_layout = HeadLayout(),
-                                     HeadLayout grad_layout = HeadLayout());
+                                     HeadLayout grad_layout = HeadLayout(),
+                                     float *column_partials = nullptr);
 
 // ---- loss (loss.cu) -------------------------------------------------------
 // row_losses: scratch of `rows` floats.

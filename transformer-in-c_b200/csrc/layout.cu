@@ -234,6 +234,55 @@ __global__ void token_patch_grad_kernel(float *__restrict__ patch_grad,
     }
 }
 
+// The three gradients of the token embedding in one pass over the tokens' gradient, for
+// batches whose launches cost more than their bytes: a block has 32 columns (of four
+// floats) of the [batch, seq * d_model] matrix and eight slices of the batch, whose sums
+// are added as a tree.
+constexpr int kEmbeddingColumns = 32, kEmbeddingSlices = 8;
+constexpr size_t kEmbeddingFloats = size_t(1) << 20;
+
+__device__ __forceinline__ float4 plus(const float4 &a, const float4 &b) {
+    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+
+__global__ void __launch_bounds__(kEmbeddingColumns * kEmbeddingSlices)
+token_embedding_backward_kernel(float4 *__restrict__ patch_grad,
+                                float4 *__restrict__ cls_grad,
+                                float4 *__restrict__ positional_grad,
+                                const float4 *__restrict__ tokens_grad, unsigned batch,
+                                unsigned columns, unsigned row_vectors, bool add) {
+    __shared__ float4 sums[kEmbeddingSlices][kEmbeddingColumns];
+    grid_dependency_wait();
+    grid_dependency_release();
+    const unsigned lane = threadIdx.x % kEmbeddingColumns;
+    const unsigned slice = threadIdx.x / kEmbeddingColumns;
+    const unsigned column = blockIdx.x * kEmbeddingColumns + lane;
+    float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (column < columns) {
+        const unsigned patch_columns = columns - row_vectors;
+#pragma unroll 4
+        for (unsigned b = slice; b < batch; b += kEmbeddingSlices) {
+            const float4 v = __ldg(tokens_grad + b * columns + column);
+            sum = plus(sum, v);
+            if (column >= row_vectors) {
+                float4 *to = patch_grad + b * patch_columns + column - row_vectors;
+                *to = add ? plus(*to, v) : v;
+            }
+        }
+    }
+    sums[slice][lane] = sum;
+    __syncthreads();
+    if (slice == 0 && column < columns) {
+        const float4 total =
+            plus(plus(plus(sums[0][lane], sums[1][lane]), plus(sums[2][lane], sums[3][lane])),
+                 plus(plus(sums[4][lane], sums[5][lane]), plus(sums[6][lane], sums[7][lane])));
+        positional_grad[column] = plus(positional_grad[column], total);
+        if (column < row_vectors) {
+            cls_grad[column] = plus(cls_grad[column], total);
+        }
+    }
+}
+
 template <int V, bool kAccumulate>
 __global__ void gather_rows_kernel(const float *__restrict__ strided,
                                    float *__restrict__ compact,
@@ -342,6 +391,19 @@ void launch_token_embedding_backward(float *patch_grad, float *cls_grad,
                                      const float *tokens_grad, size_t batch,
                                      size_t seq, size_t d_model, bool add_patch,
                                      cudaStream_t stream) {
+    if (d_model % 4 == 0 && batch * seq * d_model <= kEmbeddingFloats) {
+        const unsigned columns = unsigned(seq * d_model / 4);
+        launch_chained(token_embedding_backward_kernel,
+                       (columns + kEmbeddingColumns - 1) / kEmbeddingColumns,
+                       kEmbeddingColumns * kEmbeddingSlices, 0, stream,
+                       reinterpret_cast<float4 *>(patch_grad),
+                       reinterpret_cast<float4 *>(cls_grad),
+                       reinterpret_cast<float4 *>(positional_grad),
+                       reinterpret_cast<const float4 *>(tokens_grad), unsigned(batch),
+                       columns, unsigned(d_model / 4), add_patch);
+        ++g_kernel_launches;
+        return;
+    }
     VITB200_LAUNCH_V(d_model % 4 == 0, token_patch_grad_kernel,
                      batch * (seq - 1) * d_model, patch_grad, tokens_grad,
                      batch, seq, d_model, add_patch);

@@ -18,19 +18,16 @@
 namespace vitb200 {
 namespace {
 
-__global__ void cross_entropy_rows_kernel(
+// The losses of rows `first`, `first + step`, ... (one warp), and their gradients.
+__device__ __forceinline__ void cross_entropy_rows(
     const float *__restrict__ logits, const float *__restrict__ targets,
     const float *__restrict__ class_weights, float label_smoothing,
-    float *__restrict__ logits_grad, float *__restrict__ row_losses,
-    size_t rows, size_t cols) {
-    grid_dependency_wait();
-    grid_dependency_release();
+    float *__restrict__ logits_grad, float *row_losses, size_t rows, size_t cols,
+    size_t first, size_t step) {
     const int lane = threadIdx.x & 31;
-    const size_t warp = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const size_t warps = (size_t(gridDim.x) * blockDim.x) >> 5;
     const float off = label_smoothing / float(cols);
     const float on = 1.0f - label_smoothing + off;
-    for (size_t row = warp; row < rows; row += warps) {
+    for (size_t row = first; row < rows; row += step) {
         const float *z = logits + row * cols;
         const size_t target = static_cast<size_t>(targets[row]);
         float maximum = -FLT_MAX;
@@ -62,10 +59,9 @@ __global__ void cross_entropy_rows_kernel(
     }
 }
 
-__global__ void mean_of_rows_kernel(const float *__restrict__ row_losses,
-                                    float *__restrict__ loss, size_t rows) {
-    grid_dependency_wait();
-    grid_dependency_release();
+// loss = the mean of the rows' losses, by one block.
+__device__ __forceinline__ void mean_of_rows(const float *row_losses, float *loss,
+                                             size_t rows) {
     __shared__ float partial[32];
     float sum = 0.0f;
     for (size_t i = threadIdx.x; i < rows; i += blockDim.x) {
@@ -83,6 +79,46 @@ __global__ void mean_of_rows_kernel(const float *__restrict__ row_losses,
             loss[0] = sum / float(rows);
         }
     }
+}
+
+__global__ void cross_entropy_rows_kernel(
+    const float *__restrict__ logits, const float *__restrict__ targets,
+    const float *__restrict__ class_weights, float label_smoothing,
+    float *__restrict__ logits_grad, float *__restrict__ row_losses,
+    size_t rows, size_t cols) {
+    grid_dependency_wait();
+    grid_dependency_release();
+    cross_entropy_rows(logits, targets, class_weights, label_smoothing, logits_grad,
+                       row_losses, rows, cols,
+                       (size_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5,
+                       (size_t(gridDim.x) * blockDim.x) >> 5);
+}
+
+__global__ void mean_of_rows_kernel(const float *__restrict__ row_losses,
+                                    float *__restrict__ loss, size_t rows) {
+    grid_dependency_wait();
+    grid_dependency_release();
+    mean_of_rows(row_losses, loss, rows);
+}
+
+// Both for a batch of at most kRowsOfOneBlock rows, four to a warp, and a few hundred
+// classes: one launch instead of two that take 3 us each whatever they do, with the
+// same sums in the same order.
+constexpr int kLossThreads = 1024;
+constexpr size_t kRowsOfOneBlock = 128, kLogitsOfOneBlock = 16384;
+
+__global__ void __launch_bounds__(kLossThreads)
+cross_entropy_kernel(const float *__restrict__ logits, const float *__restrict__ targets,
+                     const float *__restrict__ class_weights, float label_smoothing,
+                     float *__restrict__ logits_grad, float *__restrict__ loss,
+                     size_t rows, size_t cols) {
+    __shared__ float row_losses[kRowsOfOneBlock];
+    grid_dependency_wait();
+    grid_dependency_release();
+    cross_entropy_rows(logits, targets, class_weights, label_smoothing, logits_grad,
+                       row_losses, rows, cols, threadIdx.x >> 5, kLossThreads / 32);
+    __syncthreads();
+    mean_of_rows(row_losses, loss, rows);
 }
 
 // Row-loss scratch for launch_softmax_cross_entropy_static.  It lives in the
@@ -147,10 +183,16 @@ void launch_softmax_cross_entropy(const float *logits, const float *targets,
                                   float *logits_grad, float *row_losses,
                                   size_t rows, size_t cols,
                                   cudaStream_t stream) {
+    if (rows <= kRowsOfOneBlock && rows * cols <= kLogitsOfOneBlock) {
+        launch_chained(cross_entropy_kernel, 1, kLossThreads, 0, stream, logits, targets,
+                       class_weights, label_smoothing, logits_grad, loss, rows, cols);
+        ++g_kernel_launches;
+        return;
+    }
     launch_chained(cross_entropy_rows_kernel, stream_grid(rows * 32),
                    kStreamThreads, 0, stream, logits, targets, class_weights,
                    label_smoothing, logits_grad, row_losses, rows, cols);
-    launch_chained(mean_of_rows_kernel, 1, 1024, 0, stream, row_losses, loss,
+    launch_chained(mean_of_rows_kernel, 1, kLossThreads, 0, stream, row_losses, loss,
                    rows);
     g_kernel_launches += 2;
 }
