@@ -103,7 +103,7 @@ unsigned long long vitb200_declined_ops(const CudaBackend *backend);
 
 /* Which kernels served the contractions: matrix products launched on the
  * tcgen05 tensor cores (and how many of those with the 128 x 256 tile) or on
- * the FP32 FMA kernel since the library was loaded, and long-sequence
+ * the FP32 kernels since the library was loaded, and long-sequence
  * attention passes served by the tcgen05 kernels or by the streaming
  * mma.sync kernels since the backend was created.  Any pointer may be NULL. */
 void vitb200_kernel_path_counters(const CudaBackend *backend,
@@ -214,8 +214,9 @@ int vitb200_set_deferred_synchronize(CudaBackend *backend, int on);
 
 /* Operand precision of the dense products issued through the op table:
  * VITB200_PRECISION_AUTO (default: TF32 tensor cores for products of at least
- * 16 Mi multiply-adds whose layout TMA can describe, FP32 FMA otherwise),
- * VITB200_PRECISION_FP32 (always FP32 FMA) or VITB200_PRECISION_TF32 (tensor
+ * 16 Mi multiply-adds whose layout TMA can describe, FP32 otherwise),
+ * VITB200_PRECISION_FP32 (always FP32: FMAs, or operands split for the
+ * tensor cores with errors no larger) or VITB200_PRECISION_TF32 (tensor
  * cores wherever the layout allows).  The environment variable VITB200_GEMM
  * (fp32 | tf32) sets the same thing at start-up; -1 returns to it. */
 void vitb200_set_gemm_precision(int precision);
@@ -384,7 +385,7 @@ int vitb200_k_softmax_cross_entropy_static(
 
 /* GEMM operand precision selectors for part 2 and VITB200_GEMM. */
 #define VITB200_PRECISION_AUTO 0  /* backend default for the shape          */
-#define VITB200_PRECISION_FP32 1  /* FP32 FMA                                */
+#define VITB200_PRECISION_FP32 1  /* FP32 accuracy                           */
 #define VITB200_PRECISION_TF32 2  /* tcgen05 kind::tf32, FP32 accumulate     */
 
 #ifdef __cplusplus

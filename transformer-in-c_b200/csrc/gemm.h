@@ -2,7 +2,7 @@
 //   forward   Y[M,N]  = X[M,K] W[K,N]
 //   backward  dX[M,K] += dY[M,N] W^T ;  dW[K,N] += X^T dY
 // (reference src/ops.c:107-165).  The dispatcher picks the tensor-core kernel
-// when the shape qualifies and the FP32 FMA kernel otherwise.
+// when the shape qualifies and the FP32 kernels otherwise.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -83,7 +83,7 @@ int gemm_chosen_precision(double multiply_adds);
 // environment variable); -1 restores the default policy.
 void gemm_set_default_precision(int precision);
 // Products launched since the library was loaded: on the tensor cores, of
-// those with the 128 x 256 tile, and on the FP32 FMA kernel.
+// those with the 128 x 256 tile, and on the FP32 kernels.
 void gemm_path_counters(unsigned long long *tensor_core,
                         unsigned long long *wide_tile, unsigned long long *fma);
 

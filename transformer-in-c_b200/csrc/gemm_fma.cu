@@ -1,7 +1,7 @@
-// FP32 FMA matrix products: the exact-FP32 policy, products too small for the
-// tensor cores and layouts TMA cannot describe.  C[M,N] (+)= A[M,K] * B[K,N]
-// for the three storage forms of a product and its two gradients (reference
-// src/ops.c:123-132 and :153-163):
+// FP32 FMA matrix products: the FP32 policy (except large ones, gemm_split.cu),
+// products too small for the tensor cores and layouts TMA cannot describe.
+// C[M,N] (+)= A[M,K] * B[K,N] for the three storage forms of a product and its two
+// gradients (reference src/ops.c:123-132 and :153-163):
 //   forward        A rows with K contiguous,  B rows with N contiguous
 //   input grad     A rows with K contiguous,  B rows with K contiguous
 //   weight grad    A rows with M contiguous,  B rows with N contiguous
