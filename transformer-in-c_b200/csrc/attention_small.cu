@@ -344,10 +344,6 @@ attention_small_backward_kernel(
     int seq, float scale, bool add_q, bool add_k, bool add_v, bool recompute,
     HeadLayout in_layout, HeadLayout out_layout, HeadLayout dout_layout,
     HeadLayout grad_layout, float *__restrict__ column_partials) {
-    // Column sums of this head's dQ, dK and dV, where they are wanted: the QKV bias
-    // gradient then reads one row per sample instead of the whole projected gradient
-    // in a launch of its own.
-    __shared__ float columns[3 * HD];
     extern __shared__ __align__(16) float shared[];
     constexpr int kPitch = kTilePitch<HD>;
     constexpr bool kTwoTiles = HD < 64 && LANES > 1;   // P and dS side by side,
@@ -359,6 +355,11 @@ attention_small_backward_kernel(
     float *do_tile = v_tile + seq * kPitch;
     float *p_tile = do_tile + seq * kPitch;
     float *ds_tile = kTwoTiles ? p_tile + seq * pitch : p_tile;
+    // Column sums of this head's dQ, dK and dV, where they are wanted: the QKV bias
+    // gradient then reads one row per sample instead of the whole projected gradient
+    // in a launch of its own.  (Part of the dynamic allocation, so that fit_shared sees
+    // all that a launch takes.)
+    float *columns = ds_tile + seq * pitch;
     const size_t group = blockIdx.x;
     const size_t base = group_offset<HD>(group, seq, in_layout);
     const int part = threadIdx.x % LANES;
@@ -484,6 +485,8 @@ attention_small_backward_kernel(
     }
 }
 
+// Every byte that a launch takes is dynamic (no kernel here has static shared memory):
+// up to 48 KiB of it are open to any launch.
 template <typename Kernel>
 bool fit_shared(Kernel kernel, size_t bytes) {
     if (bytes > 226 * 1024) {
@@ -598,7 +601,8 @@ bool launch_attention_small_backward(const float *q, const float *k,
     grad_layout = resolve_layout(grad_layout, head_dim);
     const int lanes = row_lanes(groups, head_dim);
     const size_t score_tiles = two_score_tiles(head_dim, lanes) ? 2 : 1;
-    const size_t bytes = (4 * seq * (head_dim + 4) + score_tiles * seq * (seq | 1)) *
+    const size_t bytes = (4 * seq * (head_dim + 4) + score_tiles * seq * (seq | 1) +
+                          3 * head_dim) *
                          sizeof(float);
     bool launched = false;
 #define CALL(HD, LANES)                                                        \
