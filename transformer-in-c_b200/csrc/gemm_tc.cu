@@ -33,6 +33,7 @@
 // on expiry the kernel records a code in `*status` and all roles fall through
 // to the common teardown, which frees the tensor memory.
 #include "gemm_tc.h"
+#include "gemm_tc_shared.h"
 #include "kernels.h"
 #include "device_util.cuh"
 #include "shared_limit.h"
@@ -48,27 +49,13 @@
 namespace vitb200 {
 namespace {
 
-constexpr int kTileM = 128;
-constexpr int kTileN = 128;                 // narrow tiles; the wide variant is 256
-constexpr int kBlockK = 32;                 // 128 bytes of FP32 per row
 constexpr int kMmaK = 8;                    // tf32 K per instruction
-constexpr int kOperandBytes = kTileM * kBlockK * 4;   // 16 KiB
-// Upper bound on the load ring; the launch code picks the depth that fits
-// beside the epilogue staging for the chosen number of CTAs per SM.
-constexpr int kMaxStages = 8;
-constexpr int kSmemLimit = 227 * 1024 - 1024;   // leave room for static shared memory
 constexpr int kThreads = 192;
-// The tall tile has a group of four epilogue warps for each of its two
-// accumulators, so that both drain at the same time.
-constexpr int kThreadsTall = 320;
-// So do the GELU's two epilogues on the tiles that large products run on, whose warps
-// wait for memory between their arithmetic: more of them wait at a time.
+constexpr int kThreadsTall = 320;           // with two groups of epilogue warps
 template <int TILE_M, int TILE_N, int SECOND>
-constexpr bool kTwoGroups =
-    TILE_M == 256 || (TILE_N == 256 && (SECOND == 1 || SECOND == 3)) || SECOND == 4;
+constexpr bool kTwoGroups = tc_two_groups(TILE_M, TILE_N, SECOND);
 template <int TILE_M, int TILE_N, int SECOND>
 constexpr int kThreadsOf = kTwoGroups<TILE_M, TILE_N, SECOND> ? kThreadsTall : kThreads;
-constexpr int kBarrierBytes = 320;   // 2 x kMaxStages + 4 + 16 mbarriers, TMEM slot
 
 using namespace tc;
 
@@ -90,15 +77,6 @@ struct TcParams {
     int *status;              // device-visible word, 0 = ok
 };
 
-constexpr int kSecondGelu = 1;       // D = A*B + bias, D2 = gelu(D)
-constexpr int kSecondResidual = 2;   // D = A*B + bias, D2 = D + residual
-// D = (A*B) * gelu'(H): the backward pass through a GELU folded into the
-// product that computes the GELU output's gradient.  H is read through
-// map_d2 (one 32 x 32 block per accumulator block, by TMA into the block the
-// result is then staged in); there is one output.
-constexpr int kGeluSlope = 3;
-// The same with eight epilogue warps of one staging block each on the square tile.
-constexpr int kGeluSlopeEight = 4;
 template <int SECOND>
 constexpr bool kIsSlope = SECOND == kGeluSlope || SECOND == kGeluSlopeEight;
 
@@ -1095,74 +1073,28 @@ bool prepare(const TcGemm &g, int forced_narrow, long long most_ctas, TcLaunch *
     const int m_tiles = (g.m + tile_m - 1) / tile_m;
     p.m_tiles = m_tiles;
     const int tiles = m_tiles * p.n_tiles;
-    // Two persistent CTAs per SM, each with a 2-stage load ring and 32 KiB of
-    // epilogue staging (97 KiB): they interleave their MMA issue and their
-    // epilogues, and measured faster than one CTA with a 4- to 6-stage ring
-    // at every size tried (449 against 346 TFLOP/s at [100864,512]x[512,2048]).
-    // A single output can give up the second staging buffer of each epilogue
-    // warp for a third load stage: more bytes in flight, which is what the
-    // short-K, bandwidth-bound products of this model lack.
-    int staging_bytes = 2 * kOperandBytes;
-    int ctas_per_sm = 2;
-    p.stages = 2;
-    if ((!g.d2 || !g.residual) && !g.gelu_input) {
-        // (Also the GELU pair: its two outputs share each warp's block.)
-        p.stages = 3;
-        staging_bytes = kOperandBytes;
-    }
-    static const int forced_staging =
-        getenv("VITB200_TC_STAGING") ? atoi(getenv("VITB200_TC_STAGING")) : 0;
-    static const int forced_stages =
-        getenv("VITB200_TC_STAGES") ? atoi(getenv("VITB200_TC_STAGES")) : 0;
-    static const int forced_ctas =
-        getenv("VITB200_TC_CTAS") ? atoi(getenv("VITB200_TC_CTAS")) : 0;
-    if (forced_stages > 0 && forced_stages <= kMaxStages) {
-        p.stages = forced_stages;
-    }
-    if (forced_ctas > 0) {
-        ctas_per_sm = forced_ctas;
-    }
-    if (tile_n > kTileN) {
-        // One CTA per SM (it owns all of tensor memory): four 48 KiB stages
-        // and double-buffered staging, 224 KiB.
-        ctas_per_sm = 1;
-        p.stages = tile_m > kTileM ? 3 : 4;   // 64 KiB stages when the tile is tall
-        staging_bytes = 2 * kOperandBytes;
-    }
-    if (forced_staging == 1 && !(g.d2 && g.residual)) {
-        staging_bytes = kOperandBytes;
-    } else if (forced_staging == 2 || (forced_stages > 0 && forced_staging == 0)) {
-        staging_bytes = 2 * kOperandBytes;
-    }
-    const bool narrowed = tile_n < kTileN;
-    const bool spread = narrowed && forced_narrow < 0 &&
+    static const TcForced forced = []() {
+        auto number = [](const char *name) { return getenv(name) ? atoi(getenv(name)) : 0; };
+        TcForced f;
+        f.stages = number("VITB200_TC_STAGES");
+        f.staging = number("VITB200_TC_STAGING");
+        f.ctas = number("VITB200_TC_CTAS");
+        return f;
+    }();
+    const bool spread = tile_n < kTileN && forced_narrow < 0 &&
                         (long long)tiles <= (long long)device_sm_count();
-    if (narrowed && forced_stages == 0) {
-        // The ring as deep as the reduction, where a CTA has the SM to itself.
-        const int depth = spread && !g.accumulate ? kMaxStages : 4;
-        p.stages = std::max(2, std::min(depth, p.k_blocks));
+    const TcShared shared =
+        tc_shared(tile_m, tile_n, second, p.k_blocks, g.accumulate, spread, forced);
+    p.stages = shared.stages;
+    p.staging_bytes = shared.staging_bytes;
+    if (p.stages < 1) {
+        return false;
     }
-    if (g.gelu_input && tile_n > kTileN) {
-        staging_bytes = 4 * kOperandBytes;   // two blocks for each of eight warps
-        p.stages = 3;
-    } else if (g.gelu_input) {
-        staging_bytes = 2 * kOperandBytes;
-        if (p.stages > 2 && ctas_per_sm > 1 && !narrowed) {
-            p.stages = 2;
-        }
-    }
-    if (narrowed) {
-        // What fits beside the staging blocks, for one or for two CTAs per SM.
-        const int room = (spread ? kSmemLimit : kSmemLimit / 2) - staging_bytes -
-                         kBarrierBytes;
-        p.stages = std::min(p.stages, room / ((tile_m + tile_n) * kBlockK * 4));
-    }
-    p.staging_bytes = staging_bytes;
     // One or two persistent CTAs on every multiprocessor (never more than
     // the per-CTA partial rows provide for).
     const long long slots =
-        std::min<long long>({(long long)device_sm_count() * ctas_per_sm, kGemmPartialRows,
-                             most_ctas});
+        std::min<long long>({(long long)device_sm_count() * shared.ctas_per_sm,
+                             kGemmPartialRows, most_ctas});
     int splits = 1;
     if (g.accumulate) {
         splits = choose_slices(tiles, p.k_blocks, slots, nullptr);
@@ -1186,10 +1118,8 @@ bool prepare(const TcGemm &g, int forced_narrow, long long most_ctas, TcLaunch *
     // One persistent CTA per SM (the shared-memory ring fills an SM), fewer
     // when there is less work than SMs.
     const long long items = (long long)tiles * splits;
-    const int stage_bytes = (tile_m + tile_n) * kBlockK * 4;
-    const int smem_bytes = p.stages * stage_bytes + staging_bytes + kBarrierBytes;
     out->grid = unsigned(items < slots ? items : slots);
-    out->smem_bytes = smem_bytes;
+    out->smem_bytes = shared.bytes();
     out->tile = &tile;
     out->second = second;
     return true;
