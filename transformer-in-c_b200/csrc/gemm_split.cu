@@ -3,7 +3,7 @@
 //   C[M,N] (+)= A[M,K] * B[K,N]
 //
 // in the three storage forms of gemm_fma.cu, whose place it takes where the
-// product has enough 128 x 128 tiles (gemm_split_clocks).
+// product has enough 128 x 128 tiles (gemm_split_plan.h).
 //
 // Arithmetic.  A float is the sum of three bfloat16 values (8 + 8 + 8 bits, each
 // the nearest to what the ones before it leave over), so a product of two floats
@@ -38,6 +38,7 @@
 // in tensor memory.
 #include "device_util.cuh"
 #include "gemm.h"
+#include "gemm_split_plan.h"
 #include "gemm_tc.h"
 #include "kernels.h"
 #include "shared_limit.h"
@@ -52,8 +53,8 @@ namespace {
 
 using namespace tc;
 
-constexpr int kTile = 128;
-constexpr int kBlockK = 32;
+constexpr int kTile = kSplitTile;
+constexpr int kBlockK = kSplitBlockK;
 constexpr int kParts = 3;
 constexpr int kPartBytes = kTile * kBlockK * 2;             // 8 KiB
 constexpr int kOperandBytes = kParts * kPartBytes;
@@ -625,26 +626,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a,
     }
 }
 
-bool aligned16(const void *pointer) {
-    return (reinterpret_cast<uintptr_t>(pointer) & 15) == 0;
-}
-
-// Slices of the reduction: of a product that adds to C, as many as give every SM an
-// item, of four blocks at least.
-int slices_of(const FmaGemm &g) {
-    if (g.a_k) {
-        return 1;
-    }
-    const long long tiles =
-        ((g.m + kTile - 1LL) / kTile) * ((g.n + kTile - 1) / kTile);
-    const long long blocks = (g.k + kBlockK - 1) / kBlockK;
-    return int(std::max(1LL, std::min((long long)device_sm_count() / tiles, blocks / 4)));
-}
-
 }  // namespace
 
-// The busiest SM walks its blocks in 2000 clocks each; what a tile takes before its first
-// products and after its last makes up the rest.  Measured with launches back to back
+// Measured with launches back to back
 // (us; FMA kernel -> this one; 2-norm errors against 64 bits of normal values, x 1e-7):
 //   [12800,128]x[128,128]   18.0 -> 11.5 (2.0 -> 0.75), its gradients 46 -> 24
 //   [12800,128]x[128,512]   48.1 -> 21.2 (2.0 -> 0.75),               101 -> 43
@@ -654,23 +638,12 @@ int slices_of(const FmaGemm &g) {
 //   [20000,64]x[64,64]      10.9 -> 11.5, [1600,512]x[512,128] 20.3 -> 22.8: left to FMAs
 // Weight gradients 2.8 -> 1.4 to 2.0; a sum of positive terms 1.6 to 4.3 -> 0.8 to 1.1.
 double gemm_split_clocks(const FmaGemm &g) {
-    if ((!g.a_k && g.b_k) || g.lda % 4 != 0 || g.ldb % 4 != 0 || g.ldc % 4 != 0 ||
-        !aligned16(g.a) || !aligned16(g.b) || !aligned16(g.c) ||
-        (g.gelu_out && !aligned16(g.gelu_out)) ||
-        (g.gelu_input && !aligned16(g.gelu_input)) || (g.bias && !aligned16(g.bias)) ||
-        (g.column_partials && g.partial_row_limit < int(device_sm_count()))) {
-        return HUGE_VAL;
-    }
-    const long long sms = device_sm_count();
-    const long long tiles =
-        ((g.m + kTile - 1LL) / kTile) * ((g.n + kTile - 1) / kTile);
-    const long long blocks = (g.k + kBlockK - 1) / kBlockK, slices = slices_of(g);
-    const long long rounds = (tiles * slices + sms - 1) / sms;
-    return 13000.0 + 2000.0 * double(rounds * ((blocks + slices - 1) / slices));
+    return split_plan(g, int(device_sm_count())).clocks;
 }
 
 bool launch_gemm_split(const FmaGemm &g, cudaStream_t stream, int *partial_rows) {
-    if (gemm_split_clocks(g) == HUGE_VAL) {
+    const SplitPlan plan = split_plan(g, int(device_sm_count()));
+    if (plan.clocks == HUGE_VAL) {
         return false;
     }
     SplitParams p = {};
@@ -686,13 +659,12 @@ bool launch_gemm_split(const FmaGemm &g, cudaStream_t stream, int *partial_rows)
     p.lda = g.lda;
     p.ldb = g.ldb;
     p.ldc = g.ldc;
-    p.m_tiles = (g.m + kTile - 1) / kTile;
-    p.n_tiles = (g.n + kTile - 1) / kTile;
-    p.blocks = (g.k + kBlockK - 1) / kBlockK;
+    p.m_tiles = plan.m_tiles;
+    p.n_tiles = plan.n_tiles;
+    p.blocks = plan.blocks;
+    p.blocks_per_slice = plan.blocks_per_slice;
+    p.slices = plan.slices;
     p.add = g.accumulate ? 1 : 0;
-    const int slices = slices_of(g);
-    p.blocks_per_slice = (p.blocks + slices - 1) / slices;
-    p.slices = (p.blocks + p.blocks_per_slice - 1) / p.blocks_per_slice;
     const unsigned grid = unsigned(std::min<long long>(
         (long long)p.m_tiles * p.n_tiles * p.slices, device_sm_count()));
     CUtensorMap map_a, map_b, map_c, map_gelu;
