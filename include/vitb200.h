@@ -216,7 +216,8 @@ int vitb200_set_deferred_synchronize(CudaBackend *backend, int on);
  * VITB200_PRECISION_AUTO (default: TF32 tensor cores for products of at least
  * 16 Mi multiply-adds whose layout TMA can describe, FP32 otherwise),
  * VITB200_PRECISION_FP32 (always FP32: FMAs, or operands split for the
- * tensor cores with errors no larger) or VITB200_PRECISION_TF32 (tensor
+ * tensor cores with errors no larger; of operands below 2^-110 = 8e-34 the
+ * latter keep the bits down to 2^-133 only) or VITB200_PRECISION_TF32 (tensor
  * cores wherever the layout allows).  The environment variable VITB200_GEMM
  * (fp32 | tf32) sets the same thing at start-up; -1 returns to it. */
 void vitb200_set_gemm_precision(int precision);

@@ -27,7 +27,8 @@ int main() {
                 for (int form = 0; form < 8; ++form) {
                     FmaGemm g = {memory, memory, memory, m, n, k, 4, 4, 4,
                                  bool(form & 1), bool(form & 2), bool(form & 4)};
-                    const SplitPlan plan = split_plan(g, 148);
+                    const double error = (m + n + k) % 2 ? 1e9 : 0.0;   // none, or all
+                    const SplitPlan plan = split_plan(g, 148, error);
                     const bool served = plan.clocks != HUGE_VAL;
                     check(served == (g.a_k || (!g.b_k && g.accumulate)), "form", g, plan);
                     if (!served) {
@@ -39,11 +40,22 @@ int main() {
                               plan.slices * plan.blocks_per_slice >= plan.blocks &&
                               plan.blocks * kSplitBlockK >= k,
                           "slices", g, plan);
+                    check(plan.chunk == (error == 0.0 && g.accumulate &&
+                                                 plan.blocks_per_slice <= 32 ? 1 : 2),
+                          "accumulators", g, plan);
+                    // Slices are as long as the error allows.
+                    check(error > 0.0 || !g.accumulate ||
+                              plan.blocks_per_slice <= (plan.blocks <= 64    ? 16
+                                                        : plan.blocks <= 256 ? 32 : 128),
+                          "length of slices", g, plan);
+                    FmaGemm whole = g;   // a bias belongs to whole sums
+                    whole.bias = memory;
+                    check(!g.a_k || split_plan(whole, 148, 0.0).slices == 1, "bias", g, plan);
                     g.c = memory + 1;
-                    check(split_plan(g, 148).clocks == HUGE_VAL, "alignment", g, plan);
+                    check(split_plan(g, 148, error).clocks == HUGE_VAL, "alignment", g, plan);
                     g.c = memory;
                     g.ldc = 5;
-                    check(split_plan(g, 148).clocks == HUGE_VAL, "pitch", g, plan);
+                    check(split_plan(g, 148, error).clocks == HUGE_VAL, "pitch", g, plan);
                 }
             }
         }

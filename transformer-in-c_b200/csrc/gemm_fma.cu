@@ -30,6 +30,7 @@
 // one shared-memory pipe about as long as the four FMA pipes (8 x 16 values per
 // thread leave too few warps to cover the latencies: slower).
 #include "gemm.h"
+#include "gemm_split_plan.h"
 #include "kernels.h"
 #include "device_util.cuh"
 #include "shared_limit.h"
@@ -735,11 +736,14 @@ int launch_gemm_fma(const FmaGemm &g, cudaStream_t stream, int *partial_rows) {
     }
     // (Slices in a cluster keep sums of positive terms closer than anything else does.)
     const FmaPlan plan = plan_of(g);
-    if (plan.clocks > 15000.0 && !(plan.cluster && plan.slices > 1) &&
-        gemm_split_clocks(g) < plan.clocks &&
-        launch_gemm_split(g, stream, partial_rows)) {
-        ++g_fma_products;
-        return 0;
+    if (plan.clocks > 15000.0 && !(plan.cluster && plan.slices > 1)) {
+        const double error =
+            fma_error(std::min(g.k, slice_length(g.k, plan.slices)), plan.slices);
+        if (gemm_split_clocks(g, error) < plan.clocks &&
+            launch_gemm_split(g, error, stream, partial_rows)) {
+            ++g_fma_products;
+            return 0;
+        }
     }
     FmaLaunch launch;
     if (!prepare(g, plan, stream, partial_rows, &launch)) {

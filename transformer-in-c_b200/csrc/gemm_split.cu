@@ -10,15 +10,17 @@
 // is the sum of nine products of bfloat16 values, all of them exact in FP32.  The
 // three smallest (2^-24 of the largest and less) are left out, the other six are
 // tcgen05.mma kind::f16 instructions into FP32 accumulators: the largest into one
-// that lives for 64 terms (four instructions) only, the other five into one of
-// their own.  The tensor core's additions truncate, so a long-lived accumulator of
-// large terms would drift; instead each is added, rounded to nearest, to sums that
-// the epilogue threads keep in registers.  A sum over K then takes K/64 roundings
-// one after the other where a chain of FMAs takes K.  Measured errors stand at
-// gemm_split_clocks.  Exponents keep FP32's range; only terms below 1e-30 or so lose low
-// bits (their third part underflows).  An infinity has no such parts: a block of
-// the result that is not finite is computed again by FMAs, which gives what they
-// give (recompute).
+// that lives for 64 terms (four instructions) only, or for 32 (p.chunk), the other five
+// into one of their own.  The tensor core's additions truncate, so a long-lived
+// accumulator of large terms would drift; instead each is added, rounded to nearest, to
+// sums that the epilogue threads keep in registers.  A sum over K then takes K/64
+// roundings one after the other where a chain of FMAs takes K.  What this makes of the
+// errors, and where FMAs' own are smaller, is in gemm_split_plan.h.  The third part of a
+// value holds its bits down to 2^-133, so that values below 2^-110 (8e-34) lose low bits:
+// 2-norm error 7.5e-8 with operands down to 2^-108, 1.6e-7 at 2^-112, 3.5e-5 at 2^-120.
+// (Products and sums below FP32's normal range keep what FMAs keep of them.)  An
+// infinity has no such parts: a block of the result that is not finite is computed again
+// by FMAs, which gives what they give (recompute).
 //
 // What bounds it: shared memory.  A block of 128 x 128 x 32 is 12 instructions that
 // read 8 KiB of operands in 64 clocks each; its 32 KiB of floats are written by the
@@ -63,7 +65,6 @@ constexpr int kStages = 2;
 constexpr int kRawBytes = kTile * kBlockK * 4;              // an operand's floats
 constexpr int kRawStageBytes = 2 * kRawBytes;               // 32 KiB
 constexpr int kRawStages = 3;
-constexpr int kChunk = 2;        // blocks that a main accumulator lives for
 constexpr int kConverters = 8;   // warps
 constexpr int kAdders = 8;
 constexpr int kIssuer = kConverters + kAdders;              // the last warp
@@ -86,6 +87,7 @@ struct SplitParams {
     int m, n, k;
     int m_tiles, n_tiles;
     int blocks, blocks_per_slice, slices;   // of the reduction
+    int chunk;                 // blocks that a main accumulator lives for: 1 or 2
     long long lda, ldb, ldc;
     int add;                   // C += instead of C =
     int *status;
@@ -467,7 +469,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a,
                 const uint32_t stage = smem_address(smem + kPartsAt + g % kStages * kStageBytes);
                 const int position = issuing.block - issuing.item.begin;
                 const bool first = position == 0, last = issuing.block + 1 == issuing.item.end;
-                const bool chunk_first = position % kChunk == 0;
+                const bool chunk_first = (position & (p.chunk - 1)) == 0;
                 const int main = chunks & 1, rest = opened & 1;
                 bool served = true;
                 if (chunk_first) {
@@ -488,7 +490,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a,
                 multiply_parts(small, stage, 0, 1, true);
                 multiply_parts(tmem + kMainColumns + main * kTile, stage, 0, 0, !chunk_first);
                 tcgen05_commit(&bars.parts_empty[g % kStages]);
-                if (last || position % kChunk == kChunk - 1) {
+                if (last || (position & (p.chunk - 1)) == p.chunk - 1) {
                     tcgen05_commit(&bars.main_full[main]);
                     ++chunks;
                 }
@@ -577,7 +579,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a,
             for (int j = 0; j < 32; ++j) {
                 sums[0][j] = sums[1][j] = 0.0f;
             }
-            for (int first = item.begin; first < item.end && ok; first += kChunk) {
+            for (int first = item.begin; first < item.end && ok; first += p.chunk) {
                 const int main = chunks & 1;
                 ok = __all_sync(kFullMask, mbarrier_wait(&bars.main_full[main],
                                                          (chunks >> 1) & 1));
@@ -636,13 +638,15 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a,
 //   [30000,256]x[256,1024]  338 -> 127   (2.9 -> 0.81),               679 -> 259
 //   [4329,96]x[96,384]      14.9 -> 10.4 (1.8 -> 0.69)
 //   [20000,64]x[64,64]      10.9 -> 11.5, [1600,512]x[512,128] 20.3 -> 22.8: left to FMAs
-// Weight gradients 2.8 -> 1.4 to 2.0; a sum of positive terms 1.6 to 4.3 -> 0.8 to 1.1.
-double gemm_split_clocks(const FmaGemm &g) {
-    return split_plan(g, int(device_sm_count())).clocks;
+// Weight gradients 2.8 -> 1.4 to 2.0; a sum of positive terms 1.6 to 4.3 -> 0.8 to 1.1
+// (weight gradients: gemm_split_plan.h).
+double gemm_split_clocks(const FmaGemm &g, double error) {
+    return split_plan(g, int(device_sm_count()), error).clocks;
 }
 
-bool launch_gemm_split(const FmaGemm &g, cudaStream_t stream, int *partial_rows) {
-    const SplitPlan plan = split_plan(g, int(device_sm_count()));
+bool launch_gemm_split(const FmaGemm &g, double error, cudaStream_t stream,
+                       int *partial_rows) {
+    const SplitPlan plan = split_plan(g, int(device_sm_count()), error);
     if (plan.clocks == HUGE_VAL) {
         return false;
     }
@@ -664,6 +668,7 @@ bool launch_gemm_split(const FmaGemm &g, cudaStream_t stream, int *partial_rows)
     p.blocks = plan.blocks;
     p.blocks_per_slice = plan.blocks_per_slice;
     p.slices = plan.slices;
+    p.chunk = plan.chunk;
     p.add = g.accumulate ? 1 : 0;
     const unsigned grid = unsigned(std::min<long long>(
         (long long)p.m_tiles * p.n_tiles * p.slices, device_sm_count()));

@@ -360,9 +360,11 @@ struct FmaGemm {
 // thousands.  False, with nothing launched, for all others.
 bool launch_gemm_thin(const FmaGemm &gemm, cudaStream_t stream);
 // The large ones (gemm_split.cu), on the tensor cores at FP32 accuracy: how many clocks
-// one is expected to take (infinite where it is not served), and the launch.
-double gemm_split_clocks(const FmaGemm &gemm);
-bool launch_gemm_split(const FmaGemm &gemm, cudaStream_t stream, int *partial_rows);
+// one is expected to take (infinite where it is not served, or not within `error`, see
+// gemm_split_plan.h), and the launch.
+double gemm_split_clocks(const FmaGemm &gemm, double error);
+bool launch_gemm_split(const FmaGemm &gemm, double error, cudaStream_t stream,
+                       int *partial_rows);
 // *partial_rows receives the number of rows of column_partials written.
 int launch_gemm_fma(const FmaGemm &gemm, cudaStream_t stream,
                     int *partial_rows = nullptr);
