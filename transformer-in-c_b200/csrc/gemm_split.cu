@@ -19,8 +19,9 @@
 // value holds its bits down to 2^-133, so that values below 2^-110 (8e-34) lose low bits:
 // 2-norm error 7.5e-8 with operands down to 2^-108, 1.6e-7 at 2^-112, 3.5e-5 at 2^-120.
 // (Products and sums below FP32's normal range keep what FMAs keep of them.)  An
-// infinity has no such parts: a block of the result that is not finite is computed again
-// by FMAs, which gives what they give (recompute).
+// infinity has no such parts: 32 x 32 values of the result with one among them that is not
+// finite are computed again by FMAs, which gives what they give, once the CTA's products
+// are done (recompute).
 //
 // What bounds it: shared memory.  A block of 128 x 128 x 32 is 12 instructions that
 // read 8 KiB of operands in 64 clocks each; its 32 KiB of floats are written by the
@@ -236,26 +237,64 @@ __device__ __forceinline__ void multiply_parts(uint32_t accumulator, uint32_t st
     }
 }
 
-// The lane's row of 32 columns once more, by FMAs in the order of the reduction: for
-// rows with an infinity or a NaN in them.
+// 32 rows (from row0 on) x 32 columns (a lane each, from col on) once more, by FMAs in
+// the order of the reduction, a sum of 64 terms at a time, into a block of shared memory:
+// for those with an infinity or a NaN among them.  Zeros past the matrix.  The operands
+// of eight terms are requested together; rows of which only NaNs are left are done.
 template <bool A_K, bool B_K>
-__device__ __noinline__ void recompute(const SplitParams &p, int row, int col, int k_begin,
-                                       int k_end, float *sums) {
-    for (int j = 0; j < 32; ++j) {
-        float sum = 0.0f;
-        if (row < p.m && col + j < p.n) {
-            for (int k = k_begin; k < k_end; ++k) {
-                const float x = __ldg(p.a + (A_K ? row * p.lda + k : k * p.lda + row));
-                const float y =
-                    __ldg(p.b + (B_K ? (col + j) * p.ldb + k : k * p.ldb + col + j));
-                sum = fmaf(x, y, sum);
-                if (sum != sum) {
-                    break;   // not a number whatever follows
+__device__ __forceinline__ void recompute(const SplitParams &p, int row0, int col,
+                                          int k_begin, int k_end, float *block) {
+    constexpr int kRows = 4, kTerms = 8;
+    const int lane = threadIdx.x & 31;
+    const long long column = min(col + lane, p.n - 1);
+    const float *b = p.b + (B_K ? column * p.ldb : column);
+    for (int r = 0; r < 32; r += kRows) {
+        const float *a[kRows];
+        float sum[kRows], part[kRows];
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            const long long row = min(row0 + r + i, p.m - 1);
+            a[i] = p.a + (A_K ? row * p.lda : row);
+            sum[i] = part[i] = 0.0f;
+        }
+        for (int k = k_begin; k < k_end; k += kTerms) {
+            float x[kRows][kTerms], y[kTerms];
+#pragma unroll
+            for (int t = 0; t < kTerms; ++t) {
+                const long long at = min(k + t, k_end - 1);
+                y[t] = __ldg(b + (B_K ? at : at * p.ldb));
+#pragma unroll
+                for (int i = 0; i < kRows; ++i) {
+                    x[i][t] = __ldg(a[i] + (A_K ? at : at * p.lda));
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < kTerms; ++t) {
+#pragma unroll
+                for (int i = 0; i < kRows; ++i) {
+                    part[i] = k + t < k_end ? fmaf(x[i][t], y[t], part[i]) : part[i];
+                }
+            }
+            if (k % 64 == 64 - kTerms || k + kTerms >= k_end) {
+                bool numbers = false;
+#pragma unroll
+                for (int i = 0; i < kRows; ++i) {
+                    sum[i] += part[i];
+                    part[i] = 0.0f;
+                    numbers |= sum[i] == sum[i];
+                }
+                if (!__any_sync(kFullMask, numbers)) {
+                    break;
                 }
             }
         }
-        sums[j] = sum;
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            block[(r + i) * 32 + lane] =
+                col + lane < p.n && row0 + r + i < p.m ? sum[i] : 0.0f;
+        }
     }
+    __syncwarp();
 }
 
 // Four floats from column `col` of a row of n, zeros past its end.
@@ -280,37 +319,35 @@ __device__ __forceinline__ void stage_row(float *block, const float (&v)[32]) {
     }
 }
 
-// Everything between a warp's sums (32 rows, one per lane, from row0 on; 32 columns
-// from col on) and memory, through the warp's block of shared memory.
-template <bool A_K, bool B_K>
-__device__ __forceinline__ void finish(const SplitParams &p, const CUtensorMap &map_c,
-                                       const CUtensorMap &map_gelu, float *block, int row0,
-                                       int col, int k_begin, int k_end, float (&v)[32]) {
-    if (row0 >= p.m || col >= p.n) {
-        return;   // uniform across the warp
-    }
-    const int lane = threadIdx.x & 31, row = row0 + lane;
+// Whether all of a warp's sums are finite.
+__device__ __forceinline__ bool all_finite(const float (&v)[32]) {
     // Zero times a sum is zero unless the sum is infinite or not a number.
     float probe = 0.0f;
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
         probe = fmaf(v[j], 0.0f, probe);
     }
-    auto staged_read = [&]() {   // the copy engine has read the block
-        if (lane == 0) {
-            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-        }
-        __syncwarp();
-    };
-    staged_read();
-    if (probe != 0.0f) {
-        recompute<A_K, B_K>(p, row, col, k_begin, k_end, block + lane * 32);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            v[j] = block[lane * 32 + j];
-        }
+    return __all_sync(kFullMask, probe == 0.0f);
+}
+
+// The copy engine has read the warp's block.
+__device__ __forceinline__ void await_block() {
+    if ((threadIdx.x & 31) == 0) {
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
     __syncwarp();
+}
+
+// Everything between a warp's sums (32 rows, one per lane, from row0 on; 32 columns
+// from col on) and memory, through the warp's block of shared memory.
+__device__ __forceinline__ void finish(const SplitParams &p, const CUtensorMap &map_c,
+                                       const CUtensorMap &map_gelu, float *block, int row0,
+                                       int col, float (&v)[32]) {
+    if (row0 >= p.m || col >= p.n) {
+        return;   // uniform across the warp
+    }
+    const int lane = threadIdx.x & 31, row = row0 + lane;
+    await_block();
     if (p.bias) {
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
@@ -360,10 +397,29 @@ __device__ __forceinline__ void finish(const SplitParams &p, const CUtensorMap &
         for (int j = 0; j < 32; ++j) {
             v[j] = gelu_value(v[j]);
         }
-        staged_read();
+        await_block();
         stage_row(block, v);
         send(map_gelu, false);
     }
+}
+
+// The same for 32 x 32 values whose sums were not finite.
+template <bool A_K, bool B_K>
+__device__ __noinline__ void finish_again(const SplitParams &p, const CUtensorMap &map_c,
+                                          const CUtensorMap &map_gelu, float *block,
+                                          int row0, int col, int k_begin, int k_end) {
+    if (row0 >= p.m || col >= p.n) {
+        return;   // uniform across the warp
+    }
+    await_block();
+    recompute<A_K, B_K>(p, row0, col, k_begin, k_end, block);
+    float v[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+        v[j] = block[(threadIdx.x & 31) * 32 + j];
+    }
+    __syncwarp();
+    finish(p, map_c, map_gelu, block, row0, col, v);
 }
 
 // The barriers, and what each phase of them stands for.
@@ -559,6 +615,18 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a,
                                                  (warp - kConverters) * kStagingBytes);
         const uint32_t lanes = tmem + (uint32_t(32 * quarter) << 16) + kColumns * group;
         int chunks = 0, opened = 0;
+        // Halves of items that are not finite are computed again after the last one
+        // (over many rows that takes a while, which the issuer would wait for): a bit
+        // each, two per item, those of 16 items in a lane.  (Few products have more than
+        // that many items per CTA, and have them after that many.)
+        constexpr int kRemembered = 32 * 16;
+        uint32_t put_off = 0;
+        int ordinal = 0;
+        auto again = [&](const Item &item, int half) {
+            finish_again<A_K, B_K>(p, map_c, map_gelu, block, item.m0 + 32 * quarter,
+                                   item.n0 + kColumns * group + 32 * half,
+                                   item.begin * kBlockK, min(p.k, item.end * kBlockK));
+        };
         float sums[2][32];
         auto add = [&](uint32_t columns) {
 #pragma unroll
@@ -604,13 +672,34 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a,
                 mbarrier_arrive(&bars.rest_empty[rest]);
             }
             ++opened;
+            uint32_t infinite = 0;
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
-                finish<A_K, B_K>(p, map_c, map_gelu, block, item.m0 + 32 * quarter,
-                                 item.n0 + kColumns * group + 32 * half,
-                                 item.begin * kBlockK, min(p.k, item.end * kBlockK),
-                                 sums[half]);
+                if (all_finite(sums[half])) {
+                    finish(p, map_c, map_gelu, block, item.m0 + 32 * quarter,
+                           item.n0 + kColumns * group + 32 * half, sums[half]);
+                } else {
+                    infinite |= 1u << half;
+                }
             }
+            if (lane == ordinal / 16) {
+                put_off |= infinite << (2 * (ordinal % 16));
+            }
+            if (++ordinal < kRemembered && index + int(gridDim.x) < items) {
+                continue;
+            }
+            const int first = index - (ordinal - 1) * int(gridDim.x);
+            for (uint32_t left = __ballot_sync(kFullMask, put_off != 0); left;
+                 left &= left - 1) {
+                const int from = __ffs(left) - 1;
+                for (uint32_t bits = __shfl_sync(kFullMask, put_off, from); bits;
+                     bits &= bits - 1) {
+                    const int bit = __ffs(bits) - 1;
+                    again(Item(p, first + (16 * from + bit / 2) * int(gridDim.x)), bit & 1);
+                }
+            }
+            put_off = 0;
+            ordinal = 0;
         }
         if (lane == 0) {
             asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
