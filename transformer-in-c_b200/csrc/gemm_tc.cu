@@ -813,9 +813,15 @@ bool operand_map(const float *base, unsigned long long inner, unsigned long long
 
 int *status_word() {
     static int *word = []() -> int * {
+        // (The first product may be one that is being captured, in whose mode an
+        // allocation would end the capture.)
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
         int *memory = nullptr;
-        if (cudaHostAlloc(reinterpret_cast<void **>(&memory), sizeof(int),
-                          cudaHostAllocMapped) != cudaSuccess) {
+        const cudaError_t status = cudaHostAlloc(reinterpret_cast<void **>(&memory),
+                                                 sizeof(int), cudaHostAllocMapped);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (status != cudaSuccess) {
             return nullptr;
         }
         *memory = 0;
