@@ -187,17 +187,18 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
 
     if (warp == 0) {
         if (lane == 0) {
-            int fill = 0;   // k-blocks loaded so far, across items
+            // (The next copy waits for what this thread does per block: no divisions,
+            // and one branch to the copy of an operand that is stored K-major.)
+            int s = 0;             // stage of the ring, across items
+            uint32_t phase = 1;    // parity of its last release
             for (int item = cta; item < items && ok; item += ctas) {
                 const int tile = item % tiles;
                 const int m0 = (tile / p.n_tiles) * TILE_M;
                 const int n0 = (tile % p.n_tiles) * TILE_N;
                 const int kb_begin = (item / tiles) * p.k_blocks_per_split;
                 const int kb_end = min(p.k_blocks, kb_begin + p.k_blocks_per_split);
-                for (int kb = kb_begin; kb < kb_end; ++kb, ++fill) {
-                    const int s = fill % kStages;
-                    const uint32_t phase = (fill / kStages) & 1;
-                    ok = mbarrier_wait(&empty_bar[s], phase ^ 1);
+                for (int kb = kb_begin; kb < kb_end; ++kb) {
+                    ok = mbarrier_wait(&empty_bar[s], phase);
                     if (!ok) {
                         atomicExch(p.status, 1);
                         break;
@@ -206,26 +207,30 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
                     uint8_t *b_tile = a_tile + kABytes;
                     const int k0 = kb * kBlockK;
                     mbarrier_expect_tx(&full_bar[s], kStageBytes);
-                    if (p.a_blocked) {
+                    if (!p.a_mn_major) {
+                        // One box of TILE_M rows (the map's box height).
+                        tma_load_2d(a_tile, &map_a, k0, m0, &full_bar[s]);
+                    } else if (p.a_blocked) {
                         tma_load_3d(a_tile, &map_a, 0, k0, m0 / 32, &full_bar[s]);
-                    } else if (p.a_mn_major) {
+                    } else {
                         for (int j = 0; j < TILE_M / 32; ++j) {
                             tma_load_2d(a_tile + j * 4096, &map_a, m0 + 32 * j, k0,
                                         &full_bar[s]);
                         }
-                    } else {
-                        // One box of TILE_M rows (the map's box height).
-                        tma_load_2d(a_tile, &map_a, k0, m0, &full_bar[s]);
                     }
-                    if (p.b_blocked) {
+                    if (!p.b_mn_major) {
+                        tma_load_2d(b_tile, &map_b, k0, n0, &full_bar[s]);
+                    } else if (p.b_blocked) {
                         tma_load_3d(b_tile, &map_b, 0, k0, n0 / 32, &full_bar[s]);
-                    } else if (p.b_mn_major) {
+                    } else {
                         for (int j = 0; j < TILE_N / 32; ++j) {
                             tma_load_2d(b_tile + j * 4096, &map_b, n0 + 32 * j, k0,
                                         &full_bar[s]);
                         }
-                    } else {
-                        tma_load_2d(b_tile, &map_b, k0, n0, &full_bar[s]);
+                    }
+                    if (++s == kStages) {
+                        s = 0;
+                        phase ^= 1;
                     }
                 }
             }
@@ -253,7 +258,8 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
                 p.a_mn_major ? kLayoutSwizzle128Base32 : kLayoutSwizzle128;
             const uint32_t b_layout =
                 p.b_mn_major ? kLayoutSwizzle128Base32 : kLayoutSwizzle128;
-            int drain = 0;   // k-blocks consumed so far, across items
+            int s = 0;             // stage of the ring, across items
+            uint32_t phase = 0;    // parity of its next arrival
             int local = 0;   // items processed by this CTA
             for (int item = cta; item < items && ok;
                  item += ctas, ++local) {
@@ -267,9 +273,7 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
                 // the tall tile, one per 128-row half, both used by every tile.
                 const uint32_t buffer_phase =
                     kHalves == 2 ? (local & 1) : ((local >> 1) & 1);
-                for (int kb = kb_begin; kb < kb_end; ++kb, ++drain) {
-                    const int s = drain % kStages;
-                    const uint32_t phase = (drain / kStages) & 1;
+                for (int kb = kb_begin; kb < kb_end; ++kb) {
                     ok = mbarrier_wait(&full_bar[s], phase);
                     if (!ok) {
                         atomicExch(p.status, 2);
@@ -312,6 +316,10 @@ walk_product(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorM
                         break;
                     }
                     tcgen05_commit(&empty_bar[s]);
+                    if (++s == kStages) {
+                        s = 0;
+                        phase ^= 1;
+                    }
                 }
             }
         }
