@@ -981,7 +981,16 @@ bool prepare(const TcGemm &g, int forced_narrow, long long most_ctas, TcLaunch *
     const bool divides = g.n % 256 == 0 ||
                          (g.n % 128 == 0 && g.n >= 256 &&
                           (g.n >= 1024 || (!g.accumulate && g.k >= 1024)));
-    bool wide = (!g.d2 || gelu_pair) && g.k >= (g.gelu_input ? 512 : 256) && divides;
+    bool wide = (!g.d2 || gelu_pair) && g.k >= 256 && divides;
+    if (g.gelu_input) {
+        // (See the slope's variants below.  Short of 768 terms, not with the SMs' last
+        // round of tiles so empty that three quarters of all are not filled:
+        // [12800,512] onto 512 columns, 200 tiles for 148 SMs, 1.14 of the square tile.)
+        const long long sms = device_sm_count();
+        const long long tiles = ((g.m + kTileM - 1LL) / kTileM) * ((g.n + 255) / 256);
+        wide = wide && (g.k >= 768 || (g.k >= 512 && 4 * tiles >=
+                                                         3 * sms * ((tiles + sms - 1) / sms)));
+    }
     if (forced_tile == 128 || (g.d2 && !gelu_pair)) {
         wide = false;
     } else if (forced_tile == 256 && !g.d2 && !g.gelu_input) {
@@ -1041,16 +1050,25 @@ bool prepare(const TcGemm &g, int forced_narrow, long long most_ctas, TcLaunch *
     const TcTile &tile =
         kTcTiles[narrow >= 0 ? narrow : (tall ? kTall : (wide ? kWide : kSquare))];
     const int tile_m = tile.m, tile_n = tile.n;
-    // The slope on square tiles: with a short reduction the epilogue outlasts the
-    // products, and eight warps get through it sooner (us, four warps -> eight: K = 128
-    // [102400,128]x[128,512] 90 -> 81, K = 256 [100864,256]x[256,1024] 193 -> 185); with
-    // a longer one they are in the way of the products' copies (K = 384 217 -> 233,
-    // K = 512 [25216,512]x[512,2048] 137 -> 149), and from 512 on the 128 x 256 tile is
-    // the faster (137 -> 132; 384: 217 -> 252).
+    // The slope: with a short reduction the epilogue outlasts the products, and eight
+    // warps on the square tile get through it sooner; with a longer one they are in the
+    // way of the products' copies, and from 512 terms on the 128 x 256 tile is the faster.
+    // Measured over 12800 to 65600 rows and 384 to 2048 columns, medians (and extremes)
+    // of the ratios to four warps on the square tile:
+    //          eight warps          128 x 256 tile
+    //   128    0.87 (0.79 .. 0.97)  1.27 (1.18 .. 1.59)
+    //   256    0.91 (0.81 .. 0.99)  1.21 (1.14 .. 1.42)
+    //   320    0.95 (0.85 .. 1.01)  1.17 (1.06 .. 1.31)
+    //   384    0.99 (0.87 .. 1.04)  1.14 (1.02 .. 1.24)
+    //   448    1.03 (0.92 .. 1.06)  1.08 (0.96 .. 1.19)
+    //   512    1.03 (0.96 .. 1.06)  1.01 (0.94 .. 1.15)
+    //   576    1.03 (0.98 .. 1.06)  0.94 (0.88 .. 1.11)
+    //   768    1.03 (0.96 .. 1.05)  0.85 (0.80 .. 1.03)
+    //   1024   1.02 (0.98 .. 1.08)  0.83 (0.78 .. 1.03)
     const bool square = tile_m == kTileM && tile_n == kTileN;
     const int second = g.d2 ? (g.residual ? kSecondResidual : kSecondGelu)
         : !g.gelu_input     ? 0
-        : square && g.k <= 256 ? kGeluSlopeEight : kGeluSlope;
+        : square && g.k <= 320 ? kGeluSlopeEight : kGeluSlope;
     if (!tile.kernel(second)) {
         return false;
     }
