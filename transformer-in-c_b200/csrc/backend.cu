@@ -275,6 +275,16 @@ void check_launch(const char *what) {
     check(cudaGetLastError(), what);
 }
 
+// A kernel that was chosen by a rule on sizes has to run: its output has been opened
+// for it, and what stood there before is gone.
+void must_launch(bool launched, const char *what) {
+    if (!launched) {
+        check_launch(what);
+        fprintf(stderr, "vitb200: %s was refused\n", what);
+        abort();
+    }
+}
+
 cudaEvent_t take_event(CudaBackend *backend) {
     if (!backend->free_events.empty()) {
         cudaEvent_t event = backend->free_events.back();
@@ -681,11 +691,11 @@ void run_attention(CudaBackend *backend, const PendingAttention &pending,
                                       pending.scale, backend->stream,
                                       pending.in_layout, out_layout);
     } else {
-        launch_attention_small_forward(pending.q, pending.k, pending.v, nullptr,
-                                       out, groups, pending.seq,
-                                       pending.head_dim, pending.scale, false,
-                                       true, backend->stream, pending.in_layout,
-                                       out_layout);
+        must_launch(launch_attention_small_forward(
+                        pending.q, pending.k, pending.v, nullptr, out, groups,
+                        pending.seq, pending.head_dim, pending.scale, false, true,
+                        backend->stream, pending.in_layout, out_layout),
+                    "multi_head_attention");
     }
 }
 
@@ -716,13 +726,13 @@ bool run_attention_backward(CudaBackend *backend,
             pending.out_layout, pending.dout_layout, grad_layout,
             column_partials);
     } else {
-        const bool launched = launch_attention_small_backward(
-            pending.q, pending.k, pending.v, nullptr, pending.out,
-            pending.dout, dq, dk, dv, groups, pending.seq, pending.head_dim,
-            pending.scale, add_q, add_k, add_v, true, backend->stream,
-            pending.in_layout, pending.out_layout, pending.dout_layout,
-            grad_layout, column_partials);
-        partials_written = partials_written && launched;
+        must_launch(launch_attention_small_backward(
+                        pending.q, pending.k, pending.v, nullptr, pending.out,
+                        pending.dout, dq, dk, dv, groups, pending.seq,
+                        pending.head_dim, pending.scale, add_q, add_k, add_v, true,
+                        backend->stream, pending.in_layout, pending.out_layout,
+                        pending.dout_layout, grad_layout, column_partials),
+                    "multi_head_attention_backward");
     }
     return partials_written;
 }
