@@ -1,0 +1,21 @@
+"""Training steps at the sizes where small batches leave a launch of their own: the loss
+of a row per warp (32), the token embedding's gradients (256 samples), the column sums out
+of the FP32 attention kernels (296 groups, 148 of 32-wide heads, none of 64-wide ones).
+Bounds as for all FP32 steps."""
+import pytest
+
+from test_op_table_gpu import model, run, train, within
+
+pytestmark = pytest.mark.gpu
+
+
+def check(cases):
+    found = run(cases)
+    assert len(found) == len(cases)
+    for case, errors in zip(cases, found):
+        assert within(errors, 2e-5, 2e-5), (case, errors)
+
+
+@pytest.mark.parametrize("batch,classes", [(16, 1024), (17, 500), (32, 256), (32, 257), (33, 11)])
+def test_losses(batch, classes):
+    check([train(batch, model(1, 6, 3, 32, 4, 1, classes))])
