@@ -19,3 +19,10 @@ def check(cases):
 @pytest.mark.parametrize("batch,classes", [(16, 1024), (17, 500), (32, 256), (32, 257), (33, 11)])
 def test_losses(batch, classes):
     check([train(batch, model(1, 6, 3, 32, 4, 1, classes))])
+
+
+@pytest.mark.parametrize("batch,size", [(256, 6), (257, 6), (31, 72)])
+def test_token_embeddings(batch, size):
+    """On either side of 256 samples, and of a million floats (31 x 577 tokens of 64)."""
+    check([train(batch, model(1, size, 3, 32 if size == 6 else 64, 4, 1, 2),
+                 precision="fp32")])
