@@ -26,3 +26,10 @@ def test_token_embeddings(batch, size):
     """On either side of 256 samples, and of a million floats (31 x 577 tokens of 64)."""
     check([train(batch, model(1, size, 3, 32 if size == 6 else 64, 4, 1, 2),
                  precision="fp32")])
+
+
+@pytest.mark.parametrize("batch,width,heads", [
+    (148, 32, 2), (149, 32, 2), (37, 32, 4), (38, 32, 4), (74, 64, 2), (75, 64, 2), (20, 64, 1),
+    (20, 128, 2)])
+def test_attention_gradients(batch, width, heads):
+    check([train(batch, model(1, 12, 4, width, heads, 1, 3), precision="fp32")])

@@ -1630,9 +1630,16 @@ int op_split_heads_backward(void *context, vitb200_tensor *projected,
         const bool from_tc = pending.kind == 3 &&
                              tc_attention_wanted(seq, pending.head_dim);
         // (The FP32 kernels only where a launch costs more than their sums, whose
-        // shuffles take longer than a pass over the gradient once two groups per SM
-        // are at work: FP32 batch 256 2820 -> 2845 us.)
-        const bool few_groups = batch * heads <= 2 * size_t(device_sm_count());
+        // shuffles grow with the values per lane.  Us that the sums add / that a launch of
+        // its own takes behind the kernel, over 5 to 128 tokens, up to one and up to two
+        // groups per SM: 8-wide heads 0.8 / 2.7 .. 13 and 1.5 .. 3 / 3.1 .. 5, 16-wide
+        // ones 1.4 / 2.8 .. 20 and 2.8 .. 6 / 3.4 .. 12, 32-wide ones 2.6 / 2.8 .. 12 and
+        // 5.6 .. 11 / 3.3 .. 13, with the low end where tokens are few, 64-wide ones
+        // 11 / 2.7 .. 11 and 11 .. 23 / 3.4 .. 11.  Beyond two groups per SM they cost more
+        // than the pass they save: FP32 batch 256 2820 -> 2845 us.)
+        const size_t groups = batch * heads, sms = device_sm_count();
+        const bool few_groups = pending.head_dim <= 16 ? groups <= 2 * sms
+                              : pending.head_dim <= 32 && groups <= sms;
         const size_t partial_rows =
             pending.kind == 2 || (pending.kind == 1 && few_groups)
                 ? batch : (from_tc ? attention_tc_partial_rows() : 0);
