@@ -5,11 +5,12 @@
 // in the three storage forms of gemm_fma.cu, whose place it takes where the
 // product has enough 128 x 128 tiles (gemm_split_plan.h).
 //
-// Arithmetic.  A float is the sum of three bfloat16 values (8 + 8 + 8 bits, each
-// the nearest to what the ones before it leave over), so a product of two floats
-// is the sum of nine products of bfloat16 values, all of them exact in FP32.  The
-// three smallest (2^-24 of the largest and less) are left out, the other six are
-// tcgen05.mma kind::f16 instructions into FP32 accumulators: the largest into one
+// Arithmetic (after Henry, Tang and Heinecke, "Leveraging the bfloat16 Artificial
+// Intelligence Datatype For Higher-Precision Computations", 2019).  A float is the sum of
+// three bfloat16 values (8 + 8 + 8 bits, each the nearest to what the ones before it leave
+// over), so a product of two floats is the sum of nine products of bfloat16 values, all of
+// them exact in FP32.  The three smallest (2^-24 of the largest and less) are left out, the
+// other six are tcgen05.mma kind::f16 instructions into FP32 accumulators: the largest into one
 // that lives for 64 terms (four instructions) only, or for 32 (p.chunk), the other five
 // into one of their own.  The tensor core's additions truncate, so a long-lived
 // accumulator of large terms would drift; instead each is added, rounded to nearest, to
@@ -719,16 +720,16 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a,
 
 }  // namespace
 
-// Measured with launches back to back
-// (us; FMA kernel -> this one; 2-norm errors against 64 bits of normal values, x 1e-7):
-//   [12800,128]x[128,128]   18.0 -> 11.5 (2.0 -> 0.75), its gradients 46 -> 24
-//   [12800,128]x[128,512]   48.1 -> 21.2 (2.0 -> 0.75),               101 -> 43
-//   [12800,512]x[512,128]   57.1 -> 24.0 (4.1 -> 0.90),                99 -> 41
-//   [30000,256]x[256,1024]  338 -> 127   (2.9 -> 0.81),               679 -> 259
-//   [4329,96]x[96,384]      14.9 -> 10.4 (1.8 -> 0.69)
-//   [20000,64]x[64,64]      10.9 -> 11.5, [1600,512]x[512,128] 20.3 -> 22.8: left to FMAs
-// Weight gradients 2.8 -> 1.4 to 2.0; a sum of positive terms 1.6 to 4.3 -> 0.8 to 1.1
-// (weight gradients: gemm_split_plan.h).
+// Measured with launches back to back (us; FMA kernel -> this one; 2-norm errors against
+// 64 bits of normal values, x 1e-7):
+//   [12800,128]x[128,128]   16.4 -> 9.8  (2.0 -> 0.75), its gradients  44 -> 22
+//   [12800,128]x[128,512]   46.0 -> 19.3 (2.0 -> 0.75),               100 -> 41
+//   [12800,512]x[512,128]   55.5 -> 22.1 (4.0 -> 0.90),                98 -> 39
+//   [30000,256]x[256,1024]  337 -> 120   (2.9 -> 0.81),               679 -> 254
+//   [4329,96]x[96,384]      13.3 -> 8.7  (1.8 -> 0.69),                31 -> 21
+// ([20000,64]x[64,64], 9.9, and [1600,512]x[512,128], 18.6, are left to FMAs by the
+// estimate.)  Sums of positive terms 1.5 to 4.3 -> 0.7 to 0.9; what adds to C:
+// gemm_split_plan.h.
 double gemm_split_clocks(const FmaGemm &g, double error) {
     return split_plan(g, int(device_sm_count()), error).clocks;
 }

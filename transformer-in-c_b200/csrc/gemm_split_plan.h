@@ -47,8 +47,8 @@ inline SplitPlan split_plan(const FmaGemm &g, int sms, double error) {
     };
     SplitPlan plan = {};
     // (A weight gradient that is stored would have its slices overwrite one another.)
-    if ((!g.a_k && (g.b_k || !g.accumulate)) || g.lda % 4 != 0 || g.ldb % 4 != 0 ||
-        g.ldc % 4 != 0 || !aligned16(g.a) || !aligned16(g.b) || !aligned16(g.c) ||
+    if (g.k < 1 || (!g.a_k && (g.b_k || !g.accumulate)) || g.lda % 4 != 0 ||
+        g.ldb % 4 != 0 || g.ldc % 4 != 0 || !aligned16(g.a) || !aligned16(g.b) || !aligned16(g.c) ||
         (g.gelu_out && !aligned16(g.gelu_out)) ||
         (g.gelu_input && !aligned16(g.gelu_input)) || (g.bias && !aligned16(g.bias)) ||
         (g.column_partials && g.partial_row_limit < sms)) {
