@@ -30,7 +30,10 @@ int main() {
                     const double error = (m + n + k) % 2 ? 1e9 : 0.0;   // none, or all
                     const SplitPlan plan = split_plan(g, 148, error);
                     const bool served = plan.clocks != HUGE_VAL;
-                    check(served == (g.a_k || (!g.b_k && g.accumulate)), "form", g, plan);
+                    // An input gradient that adds stays within the error or is refused.
+                    check(served == (g.a_k ? !g.accumulate || error > 0.0
+                                           : !g.b_k && g.accumulate),
+                          "form", g, plan);
                     if (!served) {
                         continue;
                     }
@@ -40,8 +43,7 @@ int main() {
                               plan.slices * plan.blocks_per_slice >= plan.blocks &&
                               plan.blocks * kSplitBlockK >= k,
                           "slices", g, plan);
-                    check(plan.chunk == (error == 0.0 && g.accumulate &&
-                                                 plan.blocks_per_slice <= 32 ? 1 : 2),
+                    check(plan.chunk == (error == 0.0 && g.accumulate ? 1 : 2),
                           "accumulators", g, plan);
                     // Slices are as long as the error allows.
                     check(error > 0.0 || !g.accumulate ||

@@ -26,18 +26,22 @@ struct SplitPlan {
 inline double fma_error(double terms, int slices) {
     return 0.0207 * (terms / slices + slices);
 }
-// Split, with accumulators that live for two blocks: what the tensor core cuts off of
-// them, a rounding per accumulator and one per slice (0.83 to 1.02).
-inline double split_error(int blocks, int slices) {
-    return std::max(0.70 + 0.01 * slices, 0.42 + 0.0225 * slices) +
-           0.0235 * ((blocks + 1) / 2) / slices;
+// Split: what the tensor core cuts off of accumulators that live for `chunk` blocks, a
+// rounding per accumulator and one per slice (0.83 to 1.05).
+inline double split_error(int blocks, int slices, int chunk) {
+    return chunk == 2 ? std::max(0.70 + 0.01 * slices, 0.42 + 0.0225 * slices) +
+                            0.0235 * ((blocks + 1) / 2) / slices
+                      : std::max(0.29 + 0.01 * slices, 0.10 + 0.0225 * slices) +
+                            0.0164 * blocks / slices;
 }
 
 // A product that adds to C is cut into slices: a weight gradient into as many as give
 // every SM an item, of four blocks at least, where that stays within `error`, which is
 // that of the FMA plan it replaces.  Where it does not, accumulators live for one block
-// (half of what is cut off; 3 to 10 % slower) and slices are of at most 512 terms (1024
-// from 2048 on, 4096 from 8192 on), and fewer than 38 of a product of several tiles.
+// (half of what is cut off; 3 to 10 % slower); where that does not do either, slices are
+// of at most 512 terms (1024 from 2048 on, 4096 from 8192 on): of the cuts within `error`
+// the one that is expected to be the fastest.  Where there is none, an input gradient is
+// left to the FMAs and a weight gradient takes the cut with the smallest error.
 // Measured errors x 1e-7 (FMAs, as many slices as give every SM an item, this):
 // [512,2048] over 2048 rows 0.70, 0.86, 0.60, over 4096 0.80, 0.94, 0.65, [512,512] over
 // 1600 0.73, 0.82, 0.59, [128,512] over 10000 1.03, 1.13, 1.00.
@@ -67,18 +71,33 @@ inline SplitPlan split_plan(const FmaGemm &g, int sms, double error) {
     // (Bias, GELU and column sums belong to whole sums.)
     const bool cut = g.accumulate && !g.bias && !g.gelu_out && !g.gelu_input &&
                      !g.column_partials;
-    if (cut && split_error(each(plan.slices), plan.slices) > error) {
+    if (cut && split_error(each(plan.slices), plan.slices, 2) > error) {
+        plan.chunk = 1;
+    }
+    if (cut && split_error(each(plan.slices), plan.slices, plan.chunk) > error) {
         const int least = each(plan.blocks <= 64 ? 16 : plan.blocks <= 256 ? 32 : 128);
-        const int most = std::max(2 * least, tiles > 1 ? std::min(even, 37) : even);
-        long long shortest = 0;
-        for (int slices = least; slices <= most; ++slices) {
-            const long long rounds = (tiles * slices + sms - 1) / sms;
-            if (shortest == 0 || rounds * (each(slices) + 4) < shortest) {
-                shortest = rounds * (each(slices) + 4);
+        double shortest = 0.0, closest = 0.0;
+        int closest_slices = least;
+        for (int slices = least; slices <= std::max(2 * least, even); ++slices) {
+            const double rounds = double((tiles * slices + sms - 1) / sms);
+            const double cost = rounds * (each(slices) + 4);
+            const double off = split_error(each(slices), slices, 1);
+            if (closest == 0.0 || off < closest) {
+                closest = off;
+                closest_slices = slices;
+            }
+            if (off <= error && (shortest == 0.0 || cost < shortest)) {
+                shortest = cost;
                 plan.slices = slices;
             }
         }
-        plan.chunk = each(plan.slices) <= 32 ? 1 : 2;
+        if (shortest == 0.0) {
+            if (g.a_k) {
+                plan.clocks = HUGE_VAL;
+                return plan;
+            }
+            plan.slices = closest_slices;
+        }
     }
     plan.blocks_per_slice = each(plan.slices);
     plan.slices = (plan.blocks + plan.blocks_per_slice - 1) / plan.blocks_per_slice;
