@@ -36,9 +36,9 @@ def test_attention_gradients(batch, width, heads):
 
 
 def test_gradients_on_both_sides_of_sharing_a_launch():
-    """Input gradients whose CTAs take few and many terms beside those of the weight
+    """Input gradients whose CTAs have one and two times the terms of the weight
     gradient's, on 288 to 592 CTAs; bounds as for the products."""
-    pairs = [(50, 512, 128), (600, 96, 384), (2916, 12, 80), (850, 96, 96)]
+    pairs = [(50, 512, 128), (600, 96, 384), (5, 384, 1024)]
     apart = [(64, 1536, 128), (1182, 96, 128), (4329, 32, 256)]
     cases = [dict(kind="gradient_pair", precision="fp32", m=m, k=k, n=n)
              for m, k, n in pairs + apart]
