@@ -33,16 +33,3 @@ def test_token_embeddings(batch, size):
     (20, 128, 2)])
 def test_attention_gradients(batch, width, heads):
     check([train(batch, model(1, 12, 4, width, heads, 1, 3), precision="fp32")])
-
-
-def test_gradients_on_both_sides_of_sharing_a_launch():
-    """Input gradients whose CTAs have one and two times the terms of the weight
-    gradient's, on 288 to 592 CTAs; bounds as for the products."""
-    pairs = [(50, 512, 128), (600, 96, 384), (5, 384, 1024)]
-    apart = [(64, 1536, 128), (1182, 96, 128), (4329, 32, 256)]
-    cases = [dict(kind="gradient_pair", precision="fp32", m=m, k=k, n=n)
-             for m, k, n in pairs + apart]
-    for case, errors in zip(cases, run(cases)):
-        size = (case["m"], case["k"], case["n"])
-        assert errors.pop("kernels") == (1 if size in pairs else 2), (case, errors)
-        assert all(error <= 2e-5 for error in errors.values()), (case, errors)

@@ -778,30 +778,13 @@ int launch_gemm_fma(const FmaGemm &g, cudaStream_t stream, int *partial_rows) {
     return 0;
 }
 
-// (Two to four CTAs to an SM share its pipes: an input gradient whose CTAs take twice the
-// terms of the weight gradient's, which would come after them in a launch of their own, is
-// then held up by them.  Of 2993 sizes that fit one launch 84 are of that kind, with 0.80 to
-// 1.34 of the time of two launches ([64,1536] x [1536,128] 1.22, [1182,96] x [96,128] 1.17,
-// [4329,32] x [32,256] 1.33); the others take 0.67 on average.)
 bool gemm_fma_pairs(int m, int k, int n) {
     if (m >= 8192) {
         return false;   // from here on thin products have kernels of their own
     }
     const FmaPlan input = plan_product(m, k, n, false, true, LLONG_MAX);
     const FmaPlan weight = plan_addition(k, n, m, false);
-    if (input.tile != kSmallestTile || weight.tile != kSmallestTile) {
-        return false;
-    }
-    auto tiles = [](int rows, int cols) {
-        return ((rows + kSmallRows - 1LL) / kSmallRows) * ((cols + kSmallCols - 1) / kSmallCols);
-    };
-    const int input_terms = slice_length(n, input.slices);
-    const int weight_terms = slice_length(m, weight.slices);
-    const int weight_slices = (m + weight_terms - 1) / weight_terms;
-    const long long ctas = tiles(m, k) * input.slices + tiles(k, n) * weight_slices;
-    const long long sms = device_sm_count();
-    return !(ctas > 2 * sms && ctas <= 4 * sms && weight_slices > 1 &&
-             input_terms >= 2 * weight_terms);
+    return input.tile == kSmallestTile && weight.tile == kSmallestTile;
 }
 
 int launch_gemm_fma_pair(const FmaGemm &input, const FmaGemm &weight, cudaStream_t stream,
